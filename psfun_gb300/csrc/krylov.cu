@@ -17,7 +17,8 @@
 // then one cooperative kernel that runs modified Gram-Schmidt in one pass over
 // the basis: each CTA keeps its rows of w, and per basis vector performs the
 // update of the previous coefficient and the dot of the next one in a single
-// sweep, separated by a bounded grid barrier.  Scalars are finalised on the
+// sweep, separated by a bounded grid barrier; below 2^19 rows every step of a
+// solve in one launch with two grid barriers per step (arnoldi_cwy.cuh).  Scalars are finalised on the
 // device, so no host round trip sits inside the loop; the per-step error
 // estimate (istop = 1) is a one-CTA kernel in the same stream.
 #include <algorithm>
@@ -26,6 +27,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "fixsum.cuh"
 #include "internal.h"
 #include "persist.cuh"
 
@@ -147,9 +149,10 @@ struct EpiLzDot {
 // the grid barriers): they follow the steps as CTA 0 publishes their T
 // entries and ask them to stop (ms_monitor_cta: the shifted residuals of a
 // multi-shift solve, one block; est_monitor_cta: the a posteriori estimates of
-// istop = 1, kEstMonitors blocks taking the iterations in turn).
+// istop = 1, several blocks taking the iterations in turn).
 enum : int { LZ_PLAIN = 0, LZ_MON_SHIFTS = 1, LZ_MON_ESTIMATE = 2 };
 constexpr int kEstMonitors = 4;
+constexpr int kCwyMonitors = 16;  // beside k_ar_cwy: its steps take ~6 us, an estimate of order 17 ~60
 template <int MODE>
 constexpr int lz_monitors() {
   return MODE == LZ_PLAIN ? 0 : (MODE == LZ_MON_SHIFTS ? 1 : kEstMonitors);
@@ -166,6 +169,7 @@ struct LzMonitor {
   int ldy;
   double* scr;
   int64_t scr_stride;
+  int count;  // monitor blocks that share the iterations
 };
 __device__ __noinline__ void ms_monitor_cta(KState& st, const MsParams& mp, int i_begin, int i_end);
 __device__ __noinline__ void est_monitor_cta(KState& st, const LzMonitor& mon, int i_begin, int i_end, int r);
@@ -549,8 +553,7 @@ PSF_DEVINL void mgs_pair_sweep(double* __restrict__ wl, int nloc, int bd, double
   }
 }
 
-// One Arnoldi step i on the G blocks [0, G) of the launch (the body of
-// k_ar_mgs_sm and of each step of k_ar_persist); nb counts the grid barriers.
+// One Arnoldi step i (the body of k_ar_mgs_sm); nb counts the grid barriers.
 // Returns 0 when the step ran, 1 when the solve had stopped or stops here
 // (every block alike), -1 when a bounded wait gave up.
 PSF_DEVINL int ar_step(KState& st, int i, int chunk, unsigned& nb, const CsrDev& A, double scaling, int fuse, int G,
@@ -710,33 +713,7 @@ __global__ void __launch_bounds__(kMgsSmThreads) k_ar_mgs_sm(KState st, int i, i
   ar_step(st, i, chunk, nb, A, scaling, fuse, gridDim.x, mgs_sm);
 }
 
-// Arnoldi with istop = 1 on a small problem: every step in one cooperative
-// launch (ar_step with the fused SpMV on the first blocks, and one more grid
-// barrier per step so that the next step's SpMV reads the finished W_i and
-// s_i), the a posteriori estimates on the last kEstMonitors blocks as in the
-// Lanczos launch (est_monitor_cta).  Block 0 publishes step i as pub = i - 1
-// (the estimate of iteration i needs H(1:i, 1:i-1)) and, when the steps end,
-// steps_end = 1 + the last step published, so that no monitor waits for a
-// step that will not come.
-__global__ void __launch_bounds__(kMgsSmThreads) k_ar_persist(KState st, int chunk, CsrDev A, double scaling, int nl,
-                                                                LzMonitor mon) {
-  extern __shared__ __align__(16) double mgs_sm[];
-  KCtrl* c = st.ctrl;
-  const int G = gridDim.x - kEstMonitors, b = blockIdx.x;
-  if (b >= G) {
-    est_monitor_cta(st, mon, 1, nl + 1, b - G);
-    return;
-  }
-  unsigned nb = 0;
-  int last = 0;
-  for (int i = 2; i <= nl; ++i) {
-    if (ar_step(st, i, chunk, nb, A, scaling, 1, G, mgs_sm) != 0) break;
-    if (b == 0 && threadIdx.x == 0) st_release_gpu(&c->pub, i - 1);
-    last = i - 1;
-    if (i < nl && !grid_sync_to(&c->bar_count, (++nb) * (unsigned)G, &c->err)) break;
-  }
-  if (b == 0 && threadIdx.x == 0) st_release_gpu(&c->steps_end, last + 1);
-}
+#include "arnoldi_cwy.cuh"
 
 // A posteriori estimate of iteration i (psfun_d_arnoldi.f90:222-276,
 // psfun_d_lanczos.f90:271-324): yk = f(H(1:i-1,1:i-1)) e1,
@@ -970,7 +947,7 @@ __device__ __noinline__ void ms_monitor_cta(KState& st, const MsParams& mp, int 
 
 // The a posteriori estimates of istop = 1 (estimate_body) for the
 // iterations i = 2 .. i_end-1 of a solve, beside the steps: monitor r of
-// kEstMonitors takes the iterations first + r, first + r + kEstMonitors, ...,
+// mon.count takes the iterations first + r, first + r + mon.count, ...,
 // and estimate i waits for step i-1 to be published.  Each estimate writes
 // its own words (yk slot, error numerator and denominator: the concurrent
 // form of estimate_tail); one that converges records its iteration with
@@ -988,7 +965,7 @@ __device__ __noinline__ void est_monitor_cta(KState& st, const LzMonitor& mon, i
   KState ste = st;
   ste.fscratch = mon.scr + (size_t)r * mon.scr_stride;
   int pub = i_begin - 1;
-  for (int i = max(2, i_begin + 1) + r; i < i_end; i += kEstMonitors) {
+  for (int i = max(2, i_begin + 1) + r; i < i_end; i += mon.count) {
     if (pub < i - 1) {
       if (threadIdx.x == 0) s_pub = monitor_wait_pub_or_end(c, i - 1);
       __syncthreads();
@@ -1252,7 +1229,8 @@ static int ensure_workspace(psfun_krylov* meth, int64_t n, int nl, int phiorder)
     PSF_CUDA(cudaMemsetAsync(meth->u.ptr, 0, sizeof(double) * ldv, stream()));
   }
   const size_t ldh = (size_t)nl + 1;
-  const size_t small = ldh * ldh + 6 * (ldh + 2) + 64;
+  // H, s, rs, yk, e1, coef, then the grid sums of k_ar_cwy (all zeroed by k_reset)
+  const size_t small = ldh * ldh + 6 * (ldh + 2) + 64 + (nl <= kCwyMaxNl ? 3 * (size_t)cwy_acc_words(nl) : 0);
   PSF_TRY(meth->small.ensure(sizeof(double) * small));
   const size_t fs = fh_scratch_doubles(nl + 1, phiorder) + 4 * ldh * ldh + 8 * ldh;
   PSF_TRY(meth->scratch.ensure(sizeof(double) * fs));
@@ -1593,49 +1571,33 @@ int krylov_apply_device(psfun_krylov* meth, psfun_serial* fun, psfun_csr* a, dou
   const int m_mon = nl + 1 + (fpk.fname == FN_PHI ? fpk.phiorder + 1 : 0);
   const bool lz_mon = istop == 1 && !arnoldi && !sai && !userf &&
                       (dense_blocks(fpk, nl + 1, true) == 1 || (long)((m_mon + 3) / 4) * m_mon <= kDenseThreads);
-  // istop = 1 Arnoldi on a small problem (the SpMV fused into the step
-  // kernel, Krylov dimension <= 64): every step in one launch with the
-  // estimates on its monitor blocks (k_ar_persist), when the step blocks and
-  // the monitors fit on the GPU at once
-  bool ar_mon = false;
-  size_t ar_smem = kMgsSmFixed + sizeof(double) * (size_t)mgs_chunk;
-  if (istop == 1 && arnoldi && !sai && !userf && fuse_spmv && nl <= 64) {
-    auto co_resident = [&](size_t bytes) {
-      static size_t attr = 0;
-      if (attr < bytes &&
-          cudaFuncSetAttribute(k_ar_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess)
-        attr = bytes;
-      int per = 0;
-      const bool ok = attr >= bytes &&
-                      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_ar_persist, kMgsSmThreads, bytes) ==
-                          cudaSuccess &&
-                      per * sm_count() >= gms + kEstMonitors;
-      (void)cudaGetLastError();
-      return ok;
-    };
+  // Arnoldi below 2^19 rows of at most 64 entries: the whole solve in one
+  // launch with two grid barriers per step (k_ar_cwy), for istop = 1 with the
+  // estimates on kCwyMonitors blocks beside the steps (Krylov dimension <= 64:
+  // a larger f(H) wants a group of blocks)
+  CwyPlan cwy;
+  if (arnoldi && !sai && !userf && !prof_enabled() && (istop == 2 || nl <= 64)) {
     // room for a monitor's Pade work matrices of the largest order (its
-    // dense evaluations in shared memory), when the blocks still fit at once
+    // dense evaluations in shared memory)
     const size_t M = (size_t)nl + 1 + (fpk.fname == FN_PHI ? (size_t)max(fpk.phiorder, 1) : 0);
     const size_t mon_smem = sizeof(double) * ((fpk.fname == FN_PHI ? 6 : 5) * M * M + 64);
-    if (fh_uses_gemm(fpk) && mon_smem > ar_smem && mon_smem <= (size_t)200 * 1024 && co_resident(mon_smem)) {
-      ar_smem = mon_smem;
-      ar_mon = true;
-    } else {
-      ar_mon = co_resident(ar_smem);
-    }
+    cwy = cwy_plan(n, nl, a->max_row, istop == 1 ? kCwyMonitors : 0,
+                   istop == 1 && fh_uses_gemm(fpk) && mon_smem <= kCwySmemMax ? mon_smem : 0);
   }
+  const bool ar_mon = cwy.G > 0 && istop == 1;
   // the monitors' words: yk per iteration, error numerator and denominator
   // per iteration, a dense scratch per monitor (allocated here, before any
   // capture; 256-byte aligned regions for the complex variants' 16-byte pairs)
   double* lz_yk_all = nullptr;
   double* lz_scr = nullptr;
   int64_t lz_scr_stride = 0;
+  const int mon_count = ar_mon ? kCwyMonitors : kEstMonitors;
   if (lz_mon || ar_mon) {
     auto al32 = [](size_t d) { return (d + 31) & ~(size_t)31; };
     const size_t ldy = (size_t)nl + 1;
     lz_scr_stride = (int64_t)al32(fh_scratch_doubles(nl + 1, fp.phiorder) + 64);
     const size_t o_errn = al32((ldy + 1) * ldy), o_errd = o_errn + al32(ldy + 2), o_scr = o_errd + al32(ldy + 2);
-    PSF_TRY(meth->par.ensure(sizeof(double) * (o_scr + (size_t)kEstMonitors * lz_scr_stride + 64)));
+    PSF_TRY(meth->par.ensure(sizeof(double) * (o_scr + (size_t)mon_count * lz_scr_stride + 64)));
     double* pb = meth->par.as<double>();
     lz_yk_all = pb;
     st.errn_all = pb + o_errn;
@@ -1652,13 +1614,14 @@ int krylov_apply_device(psfun_krylov* meth, psfun_serial* fun, psfun_csr* a, dou
     mon.ldy = nl + 1;
     mon.scr = lz_scr;
     mon.scr_stride = lz_scr_stride;
+    mon.count = kEstMonitors;
     PSF_TRY(launch_lz_persist_mode<LZ_MON_ESTIMATE>(st, A, 1, nl + 1, mon, s));
     k_par_select<<<1, kDenseThreads, 0, s>>>(st, lz_yk_all, nl + 1, -1);
     count_launch();
     PSF_CUDA(cudaGetLastError());
     return PSFUN_SUCCESS;
   };
-  auto launch_ar_estimating = [&]() -> int {
+  auto launch_cwy = [&]() -> int {
     LzMonitor mon;
     memset(&mon, 0, sizeof mon);
     mon.fp = fpk;
@@ -1668,13 +1631,24 @@ int krylov_apply_device(psfun_krylov* meth, psfun_serial* fun, psfun_csr* a, dou
     mon.ldy = nl + 1;
     mon.scr = lz_scr;
     mon.scr_stride = lz_scr_stride;
-    int chunk = mgs_chunk, nl_ = nl;
+    mon.count = kCwyMonitors;
     double sc = scaling;
-    void* args[] = {(void*)&st, (void*)&chunk, (void*)&A, (void*)&sc, (void*)&nl_, (void*)&mon};
-    PSF_CUDA(cudaLaunchCooperativeKernel((void*)k_ar_persist, dim3(gms + kEstMonitors), dim3(kMgsSmThreads), args,
-                                         ar_smem, s));
-    k_par_select<<<1, kDenseThreads, 0, s>>>(st, lz_yk_all, nl + 1, -1);
-    count_launch(2);
+    // ||w|| <= |scaling| ||A||_2 ||v||, ||A||_2 <= sqrt(n) ||A||_inf; 2^ew bounds it with a bit to spare
+    const double bound = std::fabs(scaling) * a->norm_inf * std::sqrt((double)n);
+    int ew = bound > 0.0 ? (std::isfinite(bound) ? std::ilogb(bound) + 2 : 1000) : 0;
+    int monitors = istop == 1 ? kCwyMonitors : 0;
+    int chunk = cwy.chunk, rt = cwy.rt;
+    long long* acc = reinterpret_cast<long long*>(st.coef + (ldh + 2));
+    double* Lg = st.fscratch;  // free until k_final
+    void* args[] = {(void*)&st, (void*)&A,        (void*)&sc,  (void*)&chunk, (void*)&rt,
+                    (void*)&ew, (void*)&monitors, (void*)&acc, (void*)&Lg,    (void*)&mon};
+    PSF_CUDA(cudaLaunchCooperativeKernel(cwy.vs ? (void*)k_ar_cwy<true> : (void*)k_ar_cwy<false>,
+                                         dim3(cwy.G + monitors), dim3(cwy.threads), args, cwy.smem, s));
+    count_launch();
+    if (istop == 1) {
+      k_par_select<<<1, kDenseThreads, 0, s>>>(st, lz_yk_all, nl + 1, -1);
+      count_launch();
+    }
     PSF_CUDA(cudaGetLastError());
     return PSFUN_SUCCESS;
   };
@@ -1703,8 +1677,8 @@ int krylov_apply_device(psfun_krylov* meth, psfun_serial* fun, psfun_csr* a, dou
       int rc = enqueue_prologue(false);
       if (!arnoldi) {
         if (rc == PSFUN_SUCCESS) rc = lz_mon ? launch_lz_estimating() : launch_lz_persist(st, A, 1, nl + 1, s);
-      } else if (ar_mon) {
-        if (rc == PSFUN_SUCCESS) rc = launch_ar_estimating();
+      } else if (cwy.G > 0) {
+        if (rc == PSFUN_SUCCESS) rc = launch_cwy();
       } else {
         for (int i = 2; i <= nl && rc == PSFUN_SUCCESS; ++i) rc = enqueue_step(i);
       }
