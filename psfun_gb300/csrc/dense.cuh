@@ -59,6 +59,23 @@ __host__ __device__ inline size_t fh_scratch_doubles(int m, int phiorder) {
   return a > b ? a : b;
 }
 
+// What a matrix product does with its entries beside storing them, so that the
+// linear combinations of the Taylor evaluation (an elementwise pass, a block
+// barrier and an L2 round trip each) ride on the products.  X2, X3 (null: left
+// out) and Q have leading dimension m.
+enum GemmEpiKind : int {
+  EPI_NONE = 0,
+  EPI_ADD,    // C += c0 I + c1 X1 + c2 X2 + c3 X3
+  EPI_BESIDE  // Q = c4 C + c0 I + c1 X1 + c2 X2 + c3 X3
+};
+struct GemmEpi {
+  int kind = EPI_NONE;
+  int ld1 = 0;
+  const double *X1 = nullptr, *X2 = nullptr, *X3 = nullptr;
+  double* Q = nullptr;
+  double c[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+};
+
 // A group of co-resident blocks (one cooperative launch) sharing one dense
 // f(H) evaluation: block 0 runs the evaluation and posts its heavy parts
 // here, a matrix product (kind 0: each block computes a share of the
@@ -78,6 +95,7 @@ struct DenseGroup {
   double* C;
   int m, lda, ldb, ldc;
   double alpha;
+  GemmEpi epi;    // kind 0
   unsigned seq;   // jobs posted by block 0
   unsigned done;  // jobs finished by the other blocks
   int stop;       // block 0 has finished
@@ -94,7 +112,15 @@ struct DenseSmem {
   unsigned jobs;   // products posted so far (block 0, thread 0)
   double* sws;     // the block's dynamic shared memory, for a single block's work matrices
   unsigned sws_cap;  // its size in doubles (0: none)
+  // An estimate that runs beside the steps is of no use once an earlier
+  // iteration has converged: the evaluation gives up (DENSE_ABORTED) when
+  // *abort_at < abort_below.  Null: never.
+  const int* abort_at;
+  int abort_below;
+  int aborted;
 };
+
+constexpr int DENSE_ABORTED = 1 << 20;  // returned by fh_apply_cta, never a DEVERR flag
 
 // ---- real building blocks --------------------------------------------------
 
@@ -108,7 +134,7 @@ struct DenseSmem {
 // over the sub-partitions that hold them, and single entries spread them
 // over the most warps.
 PSF_DEVINL void gemm_tasks(int m, double alpha, const double* A, int lda, const double* B, int ldb, double* C,
-                           int ldc, int t0, int t1) {
+                           int ldc, const GemmEpi& ep, int t0, int t1) {
   for (int task = t0 + (int)threadIdx.x; task < t1; task += blockDim.x) {
     const int j = task / m;
     const int i = task - j * m;
@@ -143,6 +169,19 @@ PSF_DEVINL void gemm_tasks(int m, double alpha, const double* A, int lda, const 
       }
       for (; l < m; ++l) c = fma(alpha * b[l], a[(size_t)l * lda], c);
     }
+    if (ep.kind != EPI_NONE) {
+      // the smallest terms first, the identity last
+      const size_t e = i + (size_t)j * m;
+      double s = (ep.kind == EPI_BESIDE) ? ep.c[4] * c : c;
+      if (ep.X3) {
+        s = fma(ep.c[3], ep.X3[e], s);
+        s = fma(ep.c[2], ep.X2[e], s);
+      }
+      s = fma(ep.c[1], ep.X1[i + (size_t)j * ep.ld1], s);
+      if (i == j) s += ep.c[0];
+      if (ep.kind == EPI_BESIDE) ep.Q[e] = s;
+      else c = s;
+    }
     C[i + (size_t)j * ldc] = c;
   }
 }
@@ -156,7 +195,7 @@ PSF_DEVINL void gemm_share(int T, int G, int r, int* t0, int* t1) {
 
 // Block 0 posts a job to its group (all threads call it).
 PSF_DEVINL void group_post(DenseSmem& sm, int kind, int m, double alpha, const double* A, int lda, const double* B,
-                           int ldb, double* C, int ldc) {
+                           int ldb, double* C, int ldc, const GemmEpi& epi = GemmEpi()) {
   DenseGroup* g = sm.grp;
   __syncthreads();  // the block's writes of the operands precede the post
   if (threadIdx.x == 0) {
@@ -164,6 +203,7 @@ PSF_DEVINL void group_post(DenseSmem& sm, int kind, int m, double alpha, const d
     g->A = A; g->B = B; g->C = C;
     g->m = m; g->lda = lda; g->ldb = ldb; g->ldc = ldc;
     g->alpha = alpha;
+    if (kind == 0) g->epi = epi;
     sm.jobs += 1;
     __threadfence();
     atomicExch(&g->seq, sm.jobs);
@@ -193,17 +233,17 @@ PSF_DEVINL void group_wait(DenseSmem& sm) {
 // split over the group's blocks (block 0 posts the product, computes its own
 // share and waits for the others').
 PSF_DEVINL void cta_gemm(DenseSmem& sm, int m, double alpha, const double* A, int lda, const double* B, int ldb,
-                         double* C, int ldc) {
+                         double* C, int ldc, const GemmEpi& epi = GemmEpi()) {
   const int T = m * m;
   if (!sm.grp) {
-    gemm_tasks(m, alpha, A, lda, B, ldb, C, ldc, 0, T);
+    gemm_tasks(m, alpha, A, lda, B, ldb, C, ldc, epi, 0, T);
     __syncthreads();
     return;
   }
-  group_post(sm, 0, m, alpha, A, lda, B, ldb, C, ldc);
+  group_post(sm, 0, m, alpha, A, lda, B, ldb, C, ldc, epi);
   int t0, t1;
   gemm_share(T, gridDim.x, 0, &t0, &t1);
-  gemm_tasks(m, alpha, A, lda, B, ldb, C, ldc, t0, t1);
+  gemm_tasks(m, alpha, A, lda, B, ldb, C, ldc, epi, t0, t1);
   group_wait(sm);
 }
 
@@ -291,7 +331,8 @@ PSF_DEVINL void dense_helper(DenseGroup* g) {
     if (vg->kind == 0) {
       int t0, t1;
       gemm_share(m * m, gridDim.x, blockIdx.x, &t0, &t1);
-      gemm_tasks(m, vg->alpha, vg->A, vg->lda, vg->B, vg->ldb, vg->C, vg->ldc, t0, t1);
+      const GemmEpi ep = g->epi;  // written before the post that the acquire above saw
+      gemm_tasks(m, vg->alpha, vg->A, vg->lda, vg->B, vg->ldb, vg->C, vg->ldc, ep, t0, t1);
     } else if (vg->kind == 2) {
       int c0, c1;
       gemm_share(vg->ldb, gridDim.x, blockIdx.x, &c0, &c1);
@@ -323,9 +364,19 @@ PSF_DEVINL void dense_group_begin(DenseSmem& sm, DenseGroup* grp) {
     sm.jobs = 0u;
     sm.sws = nullptr;
     sm.sws_cap = 0u;
+    sm.abort_at = nullptr;
+    sm.aborted = 0;
   }
   __syncthreads();
 }
+
+// The last thread looks at the abort word before a stage of the evaluation
+// (it has the least to do there); dense_aborted after a block barrier.
+PSF_DEVINL void dense_poll_abort(DenseSmem& sm) {
+  if (threadIdx.x == blockDim.x - 1 && sm.abort_at && *(const volatile int*)sm.abort_at < sm.abort_below)
+    sm.aborted = 1;
+}
+PSF_DEVINL bool dense_aborted(const DenseSmem& sm) { return *(const volatile int*)&sm.aborted != 0; }
 
 // A block that evaluates f(H) alone may keep the work matrices of a small
 // evaluation in its dynamic shared memory (whatever the launch gave it): on
@@ -369,23 +420,51 @@ PSF_DEVINL void cta_copy(int m, const double* A, int lda, double* B, int ldb) {
   __syncthreads();
 }
 
-// max_i sum_j |A(i,j)|
+// max_i sum_j |A(i,j)|: four lanes per row, the row sums compared as the
+// integers of their bit patterns (a NaN sum is passed over, as fmax does; an
+// FP64 maximum costs ~150 clocks of the pipe).
 PSF_DEVINL double cta_norm_inf(int m, const double* A, int lda, DenseSmem& sm) {
-  double v = 0.0;
-  for (int i = threadIdx.x; i < m; i += blockDim.x) {
+  long long v = 0;
+  const int part = threadIdx.x & 3, nw = blockDim.x >> 5;
+  for (int i0 = 0; i0 < m; i0 += blockDim.x >> 2) {
+    if (i0 + ((int)threadIdx.x & ~31) / 4 >= m) break;  // warp-uniform
+    const int i = i0 + (threadIdx.x >> 2);
     double s = 0.0;
-    for (int j = 0; j < m; ++j) s += fabs(A[i + (size_t)j * lda]);
-    v = fmax(v, s);
+    if (i < m)
+      for (int j = part; j < m; j += 4) s += fabs(A[i + (size_t)j * lda]);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    const long long k = __double_as_longlong(s);
+    if (k <= 0x7ff0000000000000LL && k > v) v = k;
   }
-  return block_max(v, sm.red);
+#pragma unroll
+  for (int o = 16; o >= 4; o >>= 1) {
+    const long long u = __shfl_xor_sync(0xffffffffu, v, o);
+    v = u > v ? u : v;
+  }
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sm.red[threadIdx.x >> 5] = __longlong_as_double(v);
+  __syncthreads();
+  for (int w = 0; w < nw; ++w) {
+    const long long u = __double_as_longlong(sm.red[w]);
+    v = u > v ? u : v;
+  }
+  __syncthreads();
+  return __longlong_as_double(v);
 }
 
-// y = A x (thread per row, sum over j in order)
+// y = A x (four lanes per row; the warps without a row issue no FP64)
 PSF_DEVINL void cta_gemv(int m, const double* A, int lda, const double* x, double* y) {
-  for (int i = threadIdx.x; i < m; i += blockDim.x) {
+  const int part = threadIdx.x & 3;
+  for (int i0 = 0; i0 < m; i0 += blockDim.x >> 2) {
+    if (i0 + ((int)threadIdx.x & ~31) / 4 >= m) break;  // warp-uniform
+    const int i = i0 + (threadIdx.x >> 2);
     double s = 0.0;
-    for (int j = 0; j < m; ++j) s = fma(A[i + (size_t)j * lda], x[j], s);
-    y[i] = s;
+    if (i < m)
+      for (int j = part; j < m; j += 4) s = fma(A[i + (size_t)j * lda], x[j], s);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    if (i < m && part == 0) y[i] = s;
   }
   __syncthreads();
 }
@@ -730,21 +809,31 @@ PSF_DEVINL bool cta_fss(int n, double* a, int nb, double* b, DenseSmem& sm) {
 }
 
 // ---- DGPADM -----------------------------------------------------------------
-// expH = exp(t H), m x m, leading dimension m.  Returns 0, or DEVERR_* flags.
-PSF_DEVINL int cta_dgpadm(int ideg, int m, double t, const double* H, int ldh, double* expH, double* scratch,
-                          DenseSmem& sm) {
-  if (m < 1 || ideg < 1 || ideg > 60) return DEVERR_BADSIZE;
+// ns = (int)(log(hnorm) / log(2)) + 2, at least 0 (dgpadm.f:95): the integer
+// part of log2, truncated towards zero.  Taken from the exponent field unless
+// the mantissa is within 2^-30 of a power of two (or hnorm is not normal),
+// where the quotient of the logarithms decides.
+PSF_DEVINL int dgpadm_ns(double hnorm) {
+  const unsigned hi = (unsigned)__double2hiint(hnorm);
+  const int e = (int)(hi >> 20) - 1023;
+  const unsigned f = (hi & 0xfffffu) << 10 | (unsigned)__double2loint(hnorm) >> 22;  // top 30 bits of the mantissa
+  int ns;
+  if (e > -1023 && e < 1024 && f != 0u && f != 0x3fffffffu) ns = (e >= 0 ? e : e + 1) + 2;
+  else ns = (int)(log(hnorm) / log(2.0)) + 2;
+  return ns < 0 ? 0 : ns;
+}
+
+// The (ideg, ideg) Pade approximant of dgpadm.f:53-168 to exp(scale H)
+// (2^ns scale = t), formed in scratch; returns its matrix, or null on a zero
+// pivot of the denominator.  *put: a free matrix for the squarings.
+PSF_DEVINL double* dgpadm_pade(int ideg, int m, double scale, int ns, const double* H, int ldh, double* scratch,
+                               double** put, DenseSmem& sm) {
+  const double scale2 = scale * scale;
   const size_t mm = (size_t)m * m;
   double* h2 = scratch;
   double* slot0 = scratch + mm;
   double* slot1 = scratch + 2 * mm;
   double* slot2 = scratch + 3 * mm;
-  double hnorm = fabs(t * cta_norm_inf(m, H, ldh, sm));
-  if (hnorm == 0.0) return DEVERR_SINGULAR;  // reference: stop 'null H'
-  int ns = (int)(log(hnorm) / log(2.0)) + 2;
-  if (ns < 0) ns = 0;
-  const double scale = ldexp(t, -ns);
-  const double scale2 = scale * scale;
   if (threadIdx.x == 0) {
     sm.coef[0] = 1.0;
     for (int k = 1; k <= ideg; ++k)
@@ -777,25 +866,141 @@ PSF_DEVINL int cta_dgpadm(int ideg, int m, double t, const double* H, int ldh, d
   for (size_t e = threadIdx.x; e < mm; e += blockDim.x) q[e] -= p[e];
   __syncthreads();
   // h2 is free from here: the pivot rows and diagonal reciprocals of the solve
-  if (!(m >= 2 ? cta_lu_solve(m, m, q, m, p, m, h2, sm) : cta_gesv(m, m, q, m, p, m, sm))) return DEVERR_SINGULAR;
+  if (!(m >= 2 ? cta_lu_solve(m, m, q, m, p, m, h2, sm) : cta_gesv(m, m, q, m, p, m, sm))) return nullptr;
   for (size_t e = threadIdx.x; e < mm; e += blockDim.x) p[e] *= 2.0;
   __syncthreads();
   for (int j = threadIdx.x; j < m; j += blockDim.x) p[j + (size_t)j * m] += 1.0;
   __syncthreads();
-  double* res = p;
   if (ns == 0 && iodd == 1) {
     for (size_t e = threadIdx.x; e < mm; e += blockDim.x) p[e] = -p[e];
     __syncthreads();
-  } else {
-    double* get = p;
-    double* put = q;
-    for (int k = 0; k < ns; ++k) {
-      cta_gemm(sm, m, 1.0, get, m, get, m, put, m);
-      double* tmp = get; get = put; put = tmp;
-    }
-    res = get;
   }
-  cta_copy(m, res, m, expH, m);
+  *put = q;
+  return p;
+}
+
+// exp(scale H) by its Taylor polynomial of degree 16 (Paterson and Stockmeyer,
+// four powers: six products), for ||scale H|| <= 1/2 in the infinity norm,
+// where the remainder 2^-17 / 17! < 3e-20 is below rounding.  The (p, p) Pade
+// approximants of degree p >= 6 equal the exponential to rounding there as
+// well (remainder 2e-17 for p = 6), at the price of five products and a dense
+// solve: on one block the factorisation and the substitutions are chains of
+// ~1100 clocks per column, 42 of the 117 thousand clocks at order 17, and two
+// thirds of the time at order 80 on a group.
+// Returns exp(scale H), or without add1 exp(scale H) - I for the squarings of
+// cta_dgpadm; null when aborted.  *put: a free matrix.
+PSF_DEVINL double* dgpadm_taylor(int m, double scale, const double* H, int ldh, double* scratch, double** put,
+                                 bool add1, DenseSmem& sm) {
+  const size_t mm = (size_t)m * m;
+  double *a2 = scratch, *a3 = a2 + mm, *a4 = a3 + mm, *u = a4 + mm, *v = u + mm;
+  // 1 / k!, k = 0..16
+  constexpr double f[17] = {1.0,
+                            1.0,
+                            1.0 / 2,
+                            1.0 / 6,
+                            1.0 / 24,
+                            1.0 / 120,
+                            1.0 / 720,
+                            1.0 / 5040,
+                            1.0 / 40320,
+                            1.0 / 362880,
+                            1.0 / 3628800,
+                            1.0 / 39916800,
+                            1.0 / 479001600,
+                            1.0 / 6227020800.0,
+                            1.0 / 87178291200.0,
+                            1.0 / 1307674368000.0,
+                            1.0 / 20922789888000.0};
+  GemmEpi ep;
+  ep.X1 = H;
+  ep.ld1 = ldh;
+  ep.X2 = a2;
+  ep.X3 = a3;
+  cta_gemm(sm, m, scale * scale, H, ldh, H, ldh, a2, m);
+  dense_poll_abort(sm);
+  cta_gemm(sm, m, scale, a2, m, H, ldh, a3, m);
+  if (dense_aborted(sm)) return nullptr;
+  ep.kind = EPI_BESIDE;
+  ep.Q = u;
+  ep.c[0] = f[12]; ep.c[1] = f[13] * scale; ep.c[2] = f[14]; ep.c[3] = f[15]; ep.c[4] = f[16];
+  cta_gemm(sm, m, 1.0, a2, m, a2, m, a4, m, ep);
+  ep.kind = EPI_ADD;
+  ep.c[0] = f[8]; ep.c[1] = f[9] * scale; ep.c[2] = f[10]; ep.c[3] = f[11];
+  dense_poll_abort(sm);
+  cta_gemm(sm, m, 1.0, u, m, a4, m, v, m, ep);
+  if (dense_aborted(sm)) return nullptr;
+  ep.c[0] = f[4]; ep.c[1] = f[5] * scale; ep.c[2] = f[6]; ep.c[3] = f[7];
+  cta_gemm(sm, m, 1.0, v, m, a4, m, u, m, ep);
+  ep.c[0] = add1 ? 1.0 : 0.0; ep.c[1] = scale; ep.c[2] = f[2]; ep.c[3] = f[3];
+  cta_gemm(sm, m, 1.0, u, m, a4, m, v, m, ep);
+  *put = u;
+  return v;
+}
+
+// expH = exp(t H), m x m, leading dimension m, by scaling and squaring as in
+// dgpadm.f.  Returns 0, DENSE_ABORTED or DEVERR_* flags.  The norm's integer
+// logarithm and the scale are formed by one thread (by every warp they would
+// cost their FP64 instructions warp after warp).  With y, y = exp(t H) x (x and
+// y distinct, outside scratch) is wanted rather than expH: a single block
+// then ends with four products with a vector in place of the last two
+// squarings.
+static __device__ __noinline__ int cta_dgpadm(int ideg, int m, double t, const double* H, int ldh, double* expH,
+                                              double* scratch, DenseSmem& sm, const double* x = nullptr,
+                                              double* y = nullptr) {
+  if (m < 1 || ideg < 1 || ideg > 60) return DEVERR_BADSIZE;
+  const size_t mm = (size_t)m * m;
+  if (scratch == sm.sws && (H < sm.sws || H >= sm.sws + sm.sws_cap)) {
+    // the work matrices are in shared memory: H too
+    cta_copy(m, H, ldh, scratch + 5 * mm, m);
+    H = scratch + 5 * mm;
+    ldh = m;
+  }
+  dense_poll_abort(sm);
+  const double hnorm = fabs(t * cta_norm_inf(m, H, ldh, sm));
+  if (hnorm == 0.0) return DEVERR_SINGULAR;  // reference: stop 'null H'
+  if (threadIdx.x == 0) {
+    const int n = dgpadm_ns(hnorm);
+    sm.iv[6] = n;
+    sm.dv[4] = ldexp(t, -n);
+  }
+  __syncthreads();
+  const int ns = sm.iv[6];
+  const double scale = sm.dv[4];
+  const int left = (y && !sm.grp) ? min(ns, 2) : 0;  // squarings left to products with x
+  const int sq = ns - left;
+  // The first two squarings are those of E = exp(.) - I, E := E^2 + 2 E, which
+  // keeps the digits that I + E would round away while E is small: the error
+  // of the result against 64 bits is 2 to 6 times smaller than with squarings
+  // of exp(.) alone (orders 39 and 59, norms 8 to 3e4).
+  const int sqe = ideg >= 6 ? min(sq, 2) : 0;
+  double* put = nullptr;
+  double* get = ideg >= 6 ? dgpadm_taylor(m, scale, H, ldh, scratch, &put, sqe == 0, sm)
+                          : dgpadm_pade(ideg, m, scale, ns, H, ldh, scratch, &put, sm);
+  if (!get) return dense_aborted(sm) ? DENSE_ABORTED : DEVERR_SINGULAR;
+  for (int k = 0; k < sq; ++k) {
+    if (dense_aborted(sm)) return DENSE_ABORTED;
+    dense_poll_abort(sm);
+    GemmEpi ep;
+    if (k < sqe) {
+      ep.kind = EPI_ADD;
+      ep.X1 = get;
+      ep.ld1 = m;
+      ep.c[1] = 2.0;
+      ep.c[0] = (k + 1 == sqe) ? 1.0 : 0.0;
+    }
+    cta_gemm(sm, m, 1.0, get, m, get, m, put, m, ep);
+    double* tmp = get; get = put; put = tmp;
+  }
+  if (y) {
+    const double* v = x;
+    for (int k = 1 << left; k > 0; --k) {
+      double* o = (k == 1) ? y : (k & 1) ? put : scratch;  // both free now
+      cta_gemv(m, get, m, v, o);
+      v = o;
+    }
+  } else {
+    cta_copy(m, get, m, expH, m);
+  }
   return 0;
 }
 
@@ -1296,24 +1501,20 @@ PSF_DEVINL void cta_sym_eig(int m, const double* A, int lda, double* w, double* 
 // `tridiag` tells that H is symmetric tridiagonal (Lanczos).  x and y must not
 // alias scratch.  USERF is not handled here (its f lives on the host).
 // Returns 0 or DEVERR_* flags.
-PSF_DEVINL int fh_apply_cta(const FunParams& fp, int m, const double* H, int ldh, const double* x, double* y,
+static __device__ __noinline__ int fh_apply_cta(const FunParams& fp, int m, const double* H, int ldh, const double* x, double* y,
                             double* scratch, bool tridiag, DenseSmem& sm) {
   if (m < 1) return DEVERR_BADSIZE;
   const size_t mm = (size_t)m * m;
   {  // the Pade variants' work matrices in shared memory when they fit
     const size_t M = (size_t)m + (fp.fname == FN_PHI ? (size_t)max(fp.phiorder, 1) : 0);
-    const size_t need = (fp.fname == FN_PHI) ? 6 * M * M + 64 : 5 * mm + 64;
+    const size_t need = 6 * M * M + 2 * M + 64;
     const bool pade = (fp.fname == FN_EXP && fp.variant == VAR_GENPADE) || fp.fname == FN_PHI;
     if (pade && !sm.grp && sm.sws && need <= sm.sws_cap) scratch = sm.sws;
   }
   if (fp.fname == FN_EXP) {
     switch (fp.variant) {
       case VAR_GENPADE: {
-        double* E = scratch + 4 * mm;
-        const int rc = cta_dgpadm(fp.padedegree, m, fp.scaling, H, ldh, E, scratch, sm);
-        if (rc) return rc;
-        cta_gemv(m, E, m, x, y);
-        return 0;
+        return cta_dgpadm(fp.padedegree, m, fp.scaling, H, ldh, nullptr, scratch, sm, x, y);
       }
       case VAR_SASQ:
       case VAR_TAYLOR: {
@@ -1348,7 +1549,6 @@ PSF_DEVINL int fh_apply_cta(const FunParams& fp, int m, const double* H, int ldh
     const int M = m + k;
     const size_t MM = (size_t)M * M;
     double* aug = scratch + 5 * MM;
-    double* E = scratch + 4 * MM;
     for (size_t t = threadIdx.x; t < MM; t += blockDim.x) {
       const int j = (int)(t / M), i = (int)(t - (size_t)j * M);
       double v = 0.0;
@@ -1358,9 +1558,14 @@ PSF_DEVINL int fh_apply_cta(const FunParams& fp, int m, const double* H, int ldh
       aug[t] = v;
     }
     __syncthreads();
-    const int rc = cta_dgpadm(fp.padedegree, M, 1.0, aug, M, E, scratch, sm);
+    // the last column of exp(aug): its product with the last unit vector
+    double* xe = aug + MM;
+    double* ye = xe + M;
+    for (int i = threadIdx.x; i < M; i += blockDim.x) xe[i] = (i == M - 1) ? 1.0 : 0.0;
+    __syncthreads();
+    const int rc = cta_dgpadm(fp.padedegree, M, 1.0, aug, M, nullptr, scratch, sm, xe, ye);
     if (rc) return rc;
-    for (int i = threadIdx.x; i < m; i += blockDim.x) y[i] = E[i + (size_t)(M - 1) * M];
+    for (int i = threadIdx.x; i < m; i += blockDim.x) y[i] = ye[i];
     __syncthreads();
     return 0;
   }

@@ -781,6 +781,7 @@ __device__ void estimate_body(KState& st, const FunParams& fp, int i, double eps
   if (breakdown_ends && tridiag && c->breakdown) return;
   const int m = i - 1;
   const int rc = fh_apply_cta(fp, m, st.H, st.ldh, st.e1, st.yk, st.fscratch, tridiag != 0, sm);
+  if (rc == DENSE_ABORTED) return;
   if (rc) {
     if (threadIdx.x == 0) {
       atomicOr(&c->err, rc);
@@ -976,6 +977,11 @@ __device__ __noinline__ void est_monitor_cta(KState& st, const LzMonitor& mon, i
     const int bd = *(volatile int*)&c->bd_step;
     if (bd != 0 && bd <= i - 1) return;  // 0: no breakdown (i - 1 >= 1)
     ste.yk = mon.yk_all + (size_t)i * mon.ldy;
+    if (threadIdx.x == 0) {
+      dsm.abort_at = &c->conv_first;
+      dsm.abort_below = i;
+    }
+    __syncthreads();
     estimate_body(ste, mon.fp, i, mon.eps, mon.tridiag, dsm, false);
     __syncthreads();
     if (threadIdx.x == 0) atomicMax(&c->est_last, i);
@@ -1264,7 +1270,7 @@ static int dense_blocks(const FunParams& fp, int m, bool tridiag) {
 
 // Dynamic shared memory of a single-block dense evaluation (with the
 // kernel's static shared memory within the 48 KB that needs no opt-in): the
-// Pade variants' work matrices up to order 31 (phi's augmented order 29).
+// Pade variant's work matrices up to order 28 (phi's augmented order).
 constexpr size_t kDenseDynSmem = 40 * 1024;
 
 // A dense kernel (its last parameter the DenseGroup*, set in args) as a group
@@ -1580,7 +1586,7 @@ int krylov_apply_device(psfun_krylov* meth, psfun_serial* fun, psfun_csr* a, dou
     // room for a monitor's Pade work matrices of the largest order (its
     // dense evaluations in shared memory)
     const size_t M = (size_t)nl + 1 + (fpk.fname == FN_PHI ? (size_t)max(fpk.phiorder, 1) : 0);
-    const size_t mon_smem = sizeof(double) * ((fpk.fname == FN_PHI ? 6 : 5) * M * M + 64);
+    const size_t mon_smem = sizeof(double) * (6 * M * M + 2 * M + 64);
     cwy = cwy_plan(n, nl, a->max_row, istop == 1 ? kCwyMonitors : 0,
                    istop == 1 && fh_uses_gemm(fpk) && mon_smem <= kCwySmemMax ? mon_smem : 0);
   }
