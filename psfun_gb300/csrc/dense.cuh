@@ -371,7 +371,8 @@ PSF_DEVINL void dense_group_begin(DenseSmem& sm, DenseGroup* grp) {
 }
 
 // The last thread looks at the abort word before a stage of the evaluation
-// (it has the least to do there); dense_aborted after a block barrier.
+// (it has the least to do there); dense_aborted after a block barrier, with
+// another one before the next look-up, so that every thread reads the same.
 PSF_DEVINL void dense_poll_abort(DenseSmem& sm) {
   if (threadIdx.x == blockDim.x - 1 && sm.abort_at && *(const volatile int*)sm.abort_at < sm.abort_below)
     sm.aborted = 1;
@@ -978,8 +979,14 @@ static __device__ __noinline__ int cta_dgpadm(int ideg, int m, double t, const d
                           : dgpadm_pade(ideg, m, scale, ns, H, ldh, scratch, &put, sm);
   if (!get) return dense_aborted(sm) ? DENSE_ABORTED : DEVERR_SINGULAR;
   for (int k = 0; k < sq; ++k) {
-    if (dense_aborted(sm)) return DENSE_ABORTED;
-    dense_poll_abort(sm);
+    // looked up before one squaring and acted on after it, in turn: with the
+    // look-up of the next squaring beside it, a thread could see a word that
+    // the others' check came too early for, and leave them at their barrier
+    if (k & 1) {
+      if (dense_aborted(sm)) return DENSE_ABORTED;
+    } else {
+      dense_poll_abort(sm);
+    }
     GemmEpi ep;
     if (k < sqe) {
       ep.kind = EPI_ADD;
