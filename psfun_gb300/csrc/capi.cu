@@ -400,6 +400,7 @@ int psfun_gpu_csr_destroy(psfun_csr* a) {
   if (!a) return PSFUN_SUCCESS;
   if (a->T) psfun_gpu_csr_destroy(a->T);
   if (a->bj_val) cudaFree(a->bj_val);
+  if (a->bj_tri) cudaFree(a->bj_tri);
   if (a->bj_col) cudaFree(a->bj_col);
   if (a->bj_rowoff) cudaFree(a->bj_rowoff);
   if (a->bj_cnt) cudaFree(a->bj_cnt);

@@ -42,6 +42,7 @@ struct CgState {
   const double* dinv;
   // BJAC factors (bj_val null unless BJAC): the warp layout of psfun_csr
   const double* bj_val;
+  const uint8_t* bj_tri;
   const uint8_t* bj_col;
   const int32_t* bj_rowoff;
   const uchar2* bj_cnt;
@@ -71,6 +72,60 @@ struct EpiResid {
   }
 };
 
+// One group of tridiagonal blocks, a block per lane: z in registers, the
+// factors read kBjAhead rows ahead of their use.  What is left is the chain
+// of 3 x 32 dependent FP64 instructions per lane (~75 clocks each, and 64 of
+// its sub-partition's pipe): ~10 thousand clocks, where the general sweep
+// below waits for offsets, factors and z in local memory in turn (88 thousand
+// clocks; lognormal grid 701 x 613, 118 iterations: 7.88 -> 5.31 ms).  Returns the lane's partial r.z (the rows from
+// the last to the first).
+constexpr int kBjAhead = 8;
+PSF_DEVINL double bjac_solve_tri(const CgState& st, int64_t g, bool mine) {
+  const int lane = threadIdx.x & 31;
+  const int64_t row0 = (g * 32 + lane) * kBjacRows;
+  const int nv = mine ? (int)min((int64_t)kBjacRows, max((int64_t)0, st.n - row0)) : 0;  // rows of this lane's block
+  const double* f = st.bj_val + (int64_t)st.bj_rowoff[g * kBjacRows] * 32 + lane;  // row r: L at 64 r, U at 64 r + 32
+  const double* ud = st.bj_udinv + g * kBjacRows * 32 + lane;
+  double z[kBjacRows], w[kBjAhead], d[kBjAhead];
+  // st.r is padded to whole blocks; rows past n are not used
+#pragma unroll
+  for (int k = 0; k < kBjacRows; k += 2) {
+    const double2 v = nv > 0 ? *reinterpret_cast<const double2*>(st.r + row0 + k) : make_double2(0.0, 0.0);
+    z[k] = k < nv ? v.x : 0.0;
+    z[k + 1] = k + 1 < nv ? v.y : 0.0;
+  }
+#pragma unroll
+  for (int k = 1; k <= kBjAhead; ++k) w[k % kBjAhead] = f[64 * k];
+#pragma unroll
+  for (int k = 1; k < kBjacRows; ++k) {  // forward: unit lower L
+    const double l = w[k % kBjAhead];
+    if (k + kBjAhead < kBjacRows) w[k % kBjAhead] = f[64 * (k + kBjAhead)];
+    z[k] = fma(-l, z[k - 1], z[k]);
+  }
+  double acc = 0.0, rr[kBjAhead];
+  auto ahead = [&](int k) {
+    w[k % kBjAhead] = f[64 * k + 32];
+    d[k % kBjAhead] = ud[32 * k];
+    rr[k % kBjAhead] = k < nv ? st.r[row0 + k] : 0.0;
+  };
+#pragma unroll
+  for (int k = kBjacRows - 1; k >= kBjacRows - kBjAhead; --k) ahead(k);
+#pragma unroll
+  for (int k = kBjacRows - 1; k >= 0; --k) {  // backward: U, reciprocal pivots
+    const double u = w[k % kBjAhead], dk = d[k % kBjAhead], rk = rr[k % kBjAhead];
+    if (k >= kBjAhead) ahead(k - kBjAhead);
+    const double s = (k + 1 < kBjacRows) ? fma(-u, z[k + 1 < kBjacRows ? k + 1 : k], z[k]) : z[k];
+    z[k] = s * dk;
+    acc = fma(rk, z[k], acc);
+  }
+#pragma unroll
+  for (int k = 0; k < kBjacRows; k += 2) {
+    if (k + 1 < nv) *reinterpret_cast<double2*>(st.z + row0 + k) = make_double2(z[k], z[k + 1]);
+    else if (k < nv) st.z[row0 + k] = z[k];
+  }
+  return acc;
+}
+
 // BJAC: z = U^{-1} L^{-1} r on the diagonal blocks that start in the rows
 // [rb, re) of this CTA.  A warp takes a group of 32 consecutive blocks, one
 // per lane, so that each load of the factors is 32 consecutive values; a
@@ -87,6 +142,10 @@ PSF_DEVINL double bjac_solve_blocks(const CgState& st, int rb, int re) {
   for (int64_t g = g0 + warp; g < g1; g += nwarps) {
     const int64_t b = g * 32 + lane;
     const bool mine = b >= kb0 && b < kb1;
+    if (st.bj_tri[g]) {
+      acc += bjac_solve_tri(st, g, mine);
+      continue;
+    }
     const int64_t row0 = b * kBjacRows;
     double zl[kBjacRows];
 #pragma unroll
@@ -170,6 +229,9 @@ __global__ void k_diag_inv(int64_t n, const double* d, double* out) {
 // returns when the stopping rule holds, itx reaches itmax, or a breakdown
 // (sigma = 0 or rho_old = 0) asks the host to restart.
 // ---------------------------------------------------------------------------
+// BJ: with the BJAC solves (their registers would cost the other
+// preconditioners 3%, and as a function call 50%).
+template <bool BJ>
 __global__ void __launch_bounds__(kSpmvThreads) k_cg_persist(CgState st, CsrDev A, int tiles_per_cta) {
   extern __shared__ __align__(128) unsigned char cg_smem_raw[];
   LzSmem& sm = *reinterpret_cast<LzSmem*>(cg_smem_raw);
@@ -191,7 +253,7 @@ __global__ void __launch_bounds__(kSpmvThreads) k_cg_persist(CgState st, CsrDev 
   auto drain = [&]() { pipe_drain(sm, pc, passes * (unsigned)(t1 - t0)); };
   auto gsync = [&]() -> bool { return grid_sync_to(&c->bar, (++nb) * (unsigned)G, &c->err); };
   const int bd = blockDim.x;
-  const bool bj = st.bj_val != nullptr;
+  constexpr bool bj = BJ;
   // ---- restart: r = b - eta A x - zeta x ; z = D r ; rho = r.z (:256-260)
   {
     EpiResid epi{&st, 0.0};
@@ -203,7 +265,7 @@ __global__ void __launch_bounds__(kSpmvThreads) k_cg_persist(CgState st, CsrDev 
     if (!bj) block_sum_store_512(epi.acc, sm.vals, sm.red, &part[bid]);
   }
   if (!gsync()) { drain(); return; }
-  if (bj) {  // z = M^{-1} r once r is complete, then rho = r.z
+  if constexpr (BJ) {  // z = M^{-1} r once r is complete, then rho = r.z
     block_sum_store_512(bjac_solve_blocks(st, rb, re), sm.vals, sm.red, &part[bid]);
     if (!gsync()) { drain(); return; }
   }
@@ -330,7 +392,7 @@ __global__ void __launch_bounds__(kSpmvThreads) k_cg_persist(CgState st, CsrDev 
       block_sum_store_512(a_r, sm.vals, sm.red, &part[3 * G + bid]);
     }
     if (!gsync()) { drain(); return; }
-    if (bj) {  // z = M^{-1} r once r is complete, then the partial r.z
+    if constexpr (BJ) {  // z = M^{-1} r once r is complete, then the partial r.z
       __syncthreads();  // the norm reductions above are done with vals/red
       block_sum_store_512(bjac_solve_blocks(st, rb, re), sm.vals, sm.red, &part[2 * G + bid]);
       if (!gsync()) { drain(); return; }
@@ -493,9 +555,21 @@ int csr_build_bjac(psfun_csr* a) {
   const int64_t nblk = (n + kBjacRows - 1) / kBjacRows, ngrp = (nblk + 31) / 32;
   std::vector<int32_t> rowoff((size_t)ngrp * kBjacRows);
   std::vector<uchar2> cnt((size_t)ngrp * kBjacRows);
+  std::vector<uint8_t> tri((size_t)std::max<int64_t>(ngrp, 1), 1);
   int64_t slots = 0;
-  for (int64_t g = 0; g < ngrp; ++g)
+  const bool tri_fits = ngrp * 2 * kBjacRows * 32 <= 0x7fffffffLL;
+  for (int64_t g = 0; g < ngrp; ++g) {
+    if (!tri_fits) tri[g] = 0;
+    for (int64_t i = g * 32 * kBjacRows; i < std::min<int64_t>(n, (g + 1) * 32 * kBjacRows); ++i)
+      for (int32_t k = birp[i]; k < birp[i + 1]; ++k)
+        if (bja[k] < i - 1 || bja[k] > i + 1) tri[g] = 0;
     for (int r = 0; r < kBjacRows; ++r) {
+      if (tri[g]) {  // one L and one U slot in every row
+        rowoff[g * kBjacRows + r] = (int32_t)slots;
+        cnt[g * kBjacRows + r] = make_uchar2(1, 1);
+        slots += 2;
+        continue;
+      }
       int ml = 0, mu = 0;
       for (int l = 0; l < 32; ++l) {
         const int64_t i = (g * 32 + l) * kBjacRows + r;
@@ -511,6 +585,7 @@ int csr_build_bjac(psfun_csr* a) {
       cnt[g * kBjacRows + r] = make_uchar2((unsigned char)ml, (unsigned char)mu);
       slots += ml + mu;
     }
+  }
   if (slots * 32 > 0x7fffffffLL) {
     set_last_error("csr_build_bjac: factors too large for 32-bit slot offsets");
     return PSFUN_ERR_INVALID_MATRIX;
@@ -543,6 +618,7 @@ int csr_build_bjac(psfun_csr* a) {
   auto fail = [&](cudaError_t e) {
     (void)cudaGetLastError();
     set_last_error(std::string("csr_build_bjac: ") + cudaGetErrorString(e));
+    cudaFree(a->bj_tri); a->bj_tri = nullptr;
     cudaFree(a->bj_val); cudaFree(a->bj_col); cudaFree(a->bj_rowoff); cudaFree(a->bj_cnt); cudaFree(a->bj_udinv);
     a->bj_val = nullptr; a->bj_col = nullptr; a->bj_rowoff = nullptr; a->bj_cnt = nullptr; a->bj_udinv = nullptr;
     return e == cudaErrorMemoryAllocation ? PSFUN_ERR_ALLOC_DEALLOC : PSFUN_ERR_CUDA;
@@ -550,6 +626,9 @@ int csr_build_bjac(psfun_csr* a) {
   cudaError_t e;
   if ((e = cudaMalloc(&a->bj_val, sizeof(double) * wval.size())) != cudaSuccess) return fail(e);
   if ((e = cudaMalloc(&a->bj_col, wcol.size())) != cudaSuccess) return fail(e);
+  if ((e = cudaMalloc(&a->bj_tri, tri.size())) != cudaSuccess) return fail(e);
+  if ((e = cudaMemcpyAsync(a->bj_tri, tri.data(), tri.size(), cudaMemcpyHostToDevice, s)) != cudaSuccess)
+    return fail(e);
   if ((e = cudaMalloc(&a->bj_rowoff, sizeof(int32_t) * rowoff.size())) != cudaSuccess) return fail(e);
   if ((e = cudaMalloc(&a->bj_cnt, sizeof(uchar2) * cnt.size())) != cudaSuccess) return fail(e);
   if ((e = cudaMalloc(&a->bj_udinv, sizeof(double) * wud.size())) != cudaSuccess) return fail(e);
@@ -641,6 +720,7 @@ int cg_device(psfun_csr* a, int prec, const double* b, double eta, double zeta, 
   st.dinv = (prec == 1) ? a->diag_inv : nullptr;
   st.bj_val = (prec == 2) ? a->bj_val : nullptr;
   st.bj_col = a->bj_col;
+  st.bj_tri = a->bj_tri;
   st.bj_rowoff = a->bj_rowoff;
   st.bj_cnt = a->bj_cnt;
   st.bj_udinv = a->bj_udinv;
@@ -675,8 +755,9 @@ int cg_device(psfun_csr* a, int prec, const double* b, double eta, double zeta, 
   count_launch(2);
   const CsrDev A = a->dev();
   // persistent grid: one block per SM, each owning a contiguous tile range
-  static int gp = 0;
-  if (!gp) gp = persist_grid_for(k_cg_persist);
+  static const int gp_plain = persist_grid_for(k_cg_persist<false>), gp_bj = persist_grid_for(k_cg_persist<true>);
+  const bool bj = st.bj_val != nullptr;
+  const int gp = bj ? gp_bj : gp_plain;
   int tpc = (A.ntiles + gp - 1) / gp;
   if (tpc < 1) tpc = 1;
   int G = (A.ntiles + tpc - 1) / tpc;
@@ -686,7 +767,8 @@ int cg_device(psfun_csr* a, int prec, const double* b, double eta, double zeta, 
     hflag[2] = 0;
     PSF_CUDA(cudaMemsetAsync(&st.c->bar, 0, sizeof(unsigned), s));
     void* args[] = {(void*)&st, (void*)&A, (void*)&tpc};
-    PSF_CUDA(cudaLaunchCooperativeKernel((void*)k_cg_persist, dim3(G), dim3(kSpmvThreads), args, kLzSmemBytes, s));
+    PSF_CUDA(cudaLaunchCooperativeKernel(bj ? (void*)k_cg_persist<true> : (void*)k_cg_persist<false>, dim3(G),
+                                         dim3(kSpmvThreads), args, kLzSmemBytes, s));
     count_launch();
     PSF_CUDA(cudaGetLastError());
     CgCtrl hc;

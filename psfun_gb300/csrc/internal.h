@@ -114,7 +114,10 @@ struct psfun_csr {
   // (bj_val: value, bj_col: column within the block; zero padding to the
   // group's longest row), bj_rowoff[32 g + r] the first slot, bj_cnt[32 g + r]
   // the L and U slot counts, bj_udinv[(32 g + r) * 32 + lane] the reciprocal
-  // pivot.
+  // pivot.  bj_tri[g]: every entry of the group lies next to the diagonal (a
+  // grid numbered along its lines): each row then has exactly one L and one U
+  // slot, so row r's are rowoff[32 g] + 2 r and the next one.
+  uint8_t* bj_tri = nullptr;
   double* bj_val = nullptr;
   uint8_t* bj_col = nullptr;
   int32_t* bj_rowoff = nullptr;
