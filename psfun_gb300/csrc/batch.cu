@@ -12,8 +12,11 @@
 //     concatenated) handed out by an atomic counter -- the device work queue --
 //     so instances of very different sizes share the GPU without idle SMs;
 //   * the last CTA to finish a phase on an instance finalises that instance's
-//     scalars in tile order (deterministic) and, after the update phase, runs
-//     the per-pair a posteriori estimate (CRAM on the tridiagonal t_k T);
+//     scalars in tile order (deterministic) and, after the update phase,
+//     publishes the step;
+//   * the per-pair a posteriori estimates (CRAM on the tridiagonal t_k T) run
+//     beside the steps, on the warps of a few monitor blocks outside the
+//     queue and the barriers (batch_monitor);
 //   * instances whose right-hand sides have all stopped leave the queue;
 //   * two bounded grid barriers per Krylov step.
 //
@@ -36,8 +39,9 @@ constexpr int kBatchMaxRhs = 4;
 constexpr int kBatchThreads = kSpmvThreads;
 constexpr int kBatchMappings = 3;  // SpMM mappings the autotuner chooses from
 
-// per-pair scalar arrays, each nl + 2 long
-enum { PA_ALPHA = 0, PA_BETA, PA_S, PA_RS, PA_YK, PA_COEF, PA_N };
+// per-pair scalar arrays, each nl + 2 long (PA_C2: beta_i s_{i-1} / s_i, the
+// factor of W_{i-1} in step i, 0 for i = 1)
+enum { PA_ALPHA = 0, PA_BETA, PA_S, PA_RS, PA_YK, PA_COEF, PA_C2, PA_N };
 
 struct PairState {
   int done;   // stopped (converged, breakdown or error)
@@ -63,7 +67,9 @@ struct BInst {
   PairState* ps; // R
   const double* X;
   double* Y;
-  unsigned* cnt;  // [0] phase tile counter, [1] active pairs
+  unsigned* cnt;  // [0] phase tile counter, [1] active pairs, [2] published steps (kPubEnd: the last)
+  int* conv;      // R: first converged iteration (2 i), or the first that met a zero pivot (2 i + 1)
+  double* est;    // R * 2 * (nl + 2): numerator and denominator of every estimate
   // quadrature item (N > 0): y = eta A Im(sum_j c_j (xi_j I + sign A)^{-1} x)
   // over the instance's Lanczos basis, in place of f(tA)x
   int N;
@@ -83,12 +89,27 @@ struct BatchArgs {
   int keeplast;
   double eps;
   unsigned* queue;  // one counter per phase, zeroed before the launch
-  unsigned* bar;    // [0] count, [1] gen
+  unsigned* bar;    // arrivals: [0] blocks that run the steps, [1] all blocks
   int* err;
   unsigned* active; // instances still running
   const int* tile_inst;  // instance of every global tile
   int chunk;             // tiles per queue grab (1..kBatchChunkMax)
+  int monitors;          // blocks of the grid that run the estimates (its last ones)
+  zc* mon_scr;           // per monitor warp: 7 R pole scratches, then R yk (batch_mon_zc)
 };
+
+constexpr unsigned kPubEnd = 0x80000000u;
+constexpr int kConvNone = 0x7f7f7f7f;  // memset of 0x7f
+// Warps of a monitor block that take estimates, one per SM sub-partition: an
+// estimate is a chain of dependent FP64 instructions on at most 28 lanes, and
+// each holds its sub-partition's pipe for 64 clocks, so that further warps
+// would only wait for one another.
+constexpr int kBatchMonWarps = 4;
+
+// Complex numbers of scratch of one monitor warp.
+__host__ __device__ inline size_t batch_mon_zc(int R, int nl) {
+  return (size_t)R * 7 * 5 * (nl + 2) + (size_t)R * ((nl + 3) / 2);
+}
 
 PSF_DEVINL double* pa(const BInst& I, int q, int which, int nl) {
   return I.scal + ((size_t)q * PA_N + which) * (size_t)(nl + 2);
@@ -202,11 +223,13 @@ PSF_DEVINL void batch_row_thread(const SpmvTile& tb, int kb, int ke, int dj, con
                                  double (&s)[R]) {
 #pragma unroll
   for (int q = 0; q < R; ++q) s[q] = 0.0;
-  int k = kb;
-  for (; k + 4 <= ke; k += 4) {
+  // the last, partial group of four is gathered at once too: entry by entry
+  // it would cost one L2 round trip each
+  for (int k = kb; k < ke; k += 4) {
     double a[4], xv[4][R];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
+      if (k + e >= ke) break;
       a[e] = tb.val[k + e];
       const double* xr = wi + (size_t)tb.ja[k + e + dj] * R;
       if (R == 4) {
@@ -223,15 +246,10 @@ PSF_DEVINL void batch_row_thread(const SpmvTile& tb, int kb, int ke, int dj, con
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
+      if (k + e >= ke) break;
 #pragma unroll
       for (int q = 0; q < R; ++q) s[q] = fma(a[e], xv[e][q], s[q]);
     }
-  }
-  for (; k < ke; ++k) {
-    const double a = tb.val[k];
-    const double* xr = wi + (size_t)tb.ja[k + dj] * R;
-#pragma unroll
-    for (int q = 0; q < R; ++q) s[q] = fma(a, __ldg(xr + q), s[q]);
   }
 }
 
@@ -382,43 +400,24 @@ PSF_DEVINL void tile_work(const BInst& I, int ph, int i, int lt, const BatchArgs
     if (threadIdx.x == 0) sm.phase[bufi] ^= 1u;
     return;
   }
-  if (ph == PH_UPDATE) {
-    const double* __restrict__ wm = (i >= 2) ? I.V + (size_t)(i - 2) * I.ldv : wi;
-    double* __restrict__ wo = I.V + (size_t)i * I.ldv;
-    double c1[R], c2[R];
-    int k2[R];
-    bool live[R];
+  // PH_RECOMB: Y[q*n + r] = sum_j coef_{q,j} W_j[r*R + q], one element of the
+  // interleaved rows per thread (consecutive loads), four in flight
+  for (int e = threadIdx.x; e < nr * R; e += blockDim.x) {
+    const int lr = e / R, q = e - lr * R;
+    const int nt = I.ps[q].nterms;
+    const double* cf = pa(I, q, PA_COEF, B.nl);
+    const double* v = I.V + (size_t)ti.r0 * R + e;
+    double acc = 0.0;
+    int j = 0;
+    for (; j + 4 <= nt; j += 4) {
+      double w[4];
 #pragma unroll
-    for (int q = 0; q < R; ++q) {
-      const double sc = pa(I, q, PA_S, B.nl)[i];
-      c1[q] = pa(I, q, PA_ALPHA, B.nl)[i];
-      c2[q] = (i >= 2) ? pa(I, q, PA_BETA, B.nl)[i] * pa(I, q, PA_S, B.nl)[i - 1] / sc : 0.0;
-      k2[q] = ilog2_normal(sc);
-      live[q] = !I.ps[q].done;
-    }
-    for (int lr = threadIdx.x; lr < nr; lr += blockDim.x) {
-      const size_t r = (size_t)(ti.r0 + lr) * R;
+      for (int o = 0; o < 4; ++o) w[o] = v[(size_t)(j + o) * I.ldv];
 #pragma unroll
-      for (int q = 0; q < R; ++q) {
-        if (!live[q]) continue;
-        const double w = fma(-c2[q], wm[r + q], fma(-c1[q], wi[r + q], I.u[r + q]));
-        accR[q] = fma(w, w, accR[q]);
-        wo[r + q] = scale_pow2(w, k2[q]);
-      }
+      for (int o = 0; o < 4; ++o) acc = fma(cf[j + o], w[o], acc);
     }
-    return;
-  }
-  // PH_RECOMB: Y[q*n + r] = sum_j coef_{q,j} W_j[r*R + q]
-  for (int lr = threadIdx.x; lr < nr; lr += blockDim.x) {
-    const int r = ti.r0 + lr;
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      const int nt = I.ps[q].nterms;
-      const double* cf = pa(I, q, PA_COEF, B.nl);
-      double acc = 0.0;
-      for (int j = 0; j < nt; ++j) acc = fma(cf[j], I.V[(size_t)j * I.ldv + (size_t)r * R + q], acc);
-      I.Y[(size_t)q * I.n + r] = acc;
-    }
+    for (; j < nt; ++j) acc = fma(cf[j], v[(size_t)j * I.ldv], acc);
+    I.Y[(size_t)q * I.n + ti.r0 + lr] = acc;
   }
 }
 
@@ -443,7 +442,9 @@ PSF_DEVINL void finalize_quad(const BInst& I, int i, const BatchArgs& B, const d
       const double sc = pa(I, q, PA_S, nl)[i];
       const double wn = sqrt(tot[q]);
       pa(I, q, PA_BETA, nl)[i + 1] = sc * wn;
-      pa(I, q, PA_S, nl)[i + 1] = 1.0 / ldexp(wn, ilog2_normal(sc));
+      const double sn = 1.0 / ldexp(wn, ilog2_normal(sc));
+      pa(I, q, PA_S, nl)[i + 1] = sn;
+      pa(I, q, PA_C2, nl)[i + 1] = pa(I, q, PA_BETA, nl)[i + 1] * sc / sn;
       P.itx = i;
     }
   }
@@ -617,104 +618,124 @@ PSF_DEVINL void final_quad(const BInst& I, const BatchArgs& B) {
   __syncthreads();
 }
 
+// Sums of the R per-thread values over the block, into out[0..R) by the lanes
+// 0..R-1 of warp 0 (other lanes of the warp see them after a __syncwarp).
+// While a value per lane is left the lanes exchange halves of the values, so
+// that four sums take 6 FP64 instructions of each warp where one butterfly
+// per sum takes 20 (each holds its sub-partition's pipe for 64 clocks: 5100
+// against 1500 clocks for 16 warps), and the warps' sums are added by a
+// butterfly of one warp.  red holds 16 * 4 doubles; it is rewritten only
+// after the caller's next block barrier.  All threads of the block call it.
+template <int R>
+PSF_DEVINL void block_sum_R(const double* acc, double* red, double* out) {
+  constexpr int RP = (R == 3) ? 4 : R;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double v[RP];
+#pragma unroll
+  for (int q = 0; q < RP; ++q) v[q] = (q < R) ? acc[q] : 0.0;
+  int n = RP, o = 16, own = 0;  // own: the value that this lane's sum belongs to
+#pragma unroll
+  for (; n > 1; n >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int q = 0; q < RP / 2; ++q) {
+      if (q >= n / 2) break;
+      const double keep = up ? v[q + n / 2] : v[q], send = up ? v[q] : v[q + n / 2];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+    own += up ? n / 2 : 0;
+  }
+#pragma unroll
+  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  if ((lane & (32 / RP - 1)) == 0) red[wid * RP + own] = v[0];
+  __syncthreads();
+  if (wid == 0) {
+    const int tot = (int)(blockDim.x >> 5) * RP;
+    double t = 0.0;
+    for (int l = lane; l < tot; l += 32) t += red[l];
+#pragma unroll
+    for (int w = 16; w >= RP; w >>= 1) t += __shfl_xor_sync(0xffffffffu, t, w);
+    if (lane < R) out[lane] = t;
+  }
+}
+
 // Finalisation by the last CTA of an instance (deterministic tile order).
 template <int R>
-PSF_DEVINL void finalize(const BInst& I, int ph, int i, const BatchArgs& B, double* red) {
+PSF_DEVINL void finalize(const BInst& I, int ph, int i, const BatchArgs& B, double* redR) {
   const int nl = B.nl;
   const double* part = I.part + (size_t)((ph == PH_UPDATE) ? 1 : 0) * I.ntiles * R;
-  double tot[R];
+  __shared__ double tot[kBatchMaxRhs];
+  {
+    double v[R];
 #pragma unroll
-  for (int q = 0; q < R; ++q) {
-    double v = 0.0;
-    for (int t = threadIdx.x; t < I.ntiles; t += blockDim.x) v += part[(size_t)t * R + q];
-    tot[q] = block_sum(v, red);
+    for (int q = 0; q < R; ++q) v[q] = 0.0;
+    for (int t = threadIdx.x; t < I.ntiles; t += blockDim.x) {
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] += __ldcg(part + (size_t)t * R + q);
+    }
+    __syncthreads();  // redR is free
+    block_sum_R<R>(v, redR, tot);
+    __syncthreads();
   }
   if (ph == PH_INIT) {
+    if (threadIdx.x < R) {
+      const int q = threadIdx.x;
+      PairState& P = I.ps[q];
+      const double b0 = sqrt(tot[q]);
+      P.beta0 = b0;
+      pa(I, q, PA_RS, nl)[1] = b0;
+      P.errnum = 0.0;
+      P.errden = 1.0;
+      if (b0 == 0.0) { P.done = 1; P.itx = 0; }
+      else pa(I, q, PA_S, nl)[1] = 1.0 / b0;
+      __threadfence();
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
       int live = 0;
-      for (int q = 0; q < R; ++q) {
-        PairState& P = I.ps[q];
-        const double b0 = sqrt(tot[q]);
-        P.beta0 = b0;
-        pa(I, q, PA_RS, nl)[1] = b0;
-        P.errnum = 0.0;
-        P.errden = 1.0;
-        if (b0 == 0.0) { P.done = 1; P.itx = 0; }
-        else { pa(I, q, PA_S, nl)[1] = 1.0 / b0; ++live; }
-      }
+      for (int q = 0; q < R; ++q) live += !I.ps[q].done;
       I.cnt[1] = live;
-      if (live == 0) atomicSub(B.active, 1u);
+      if (live == 0) {
+        atomicSub(B.active, 1u);
+        st_release_gpu(reinterpret_cast<int*>(&I.cnt[2]), (int)kPubEnd);
+      }
     }
     return;
   }
   if (ph == PH_SPMM) {
-    if (threadIdx.x == 0) {
-      for (int q = 0; q < R; ++q) {
-        if (I.ps[q].done) continue;
+    if (threadIdx.x < R) {
+      const int q = threadIdx.x;
+      if (!I.ps[q].done) {
         const double sc = pa(I, q, PA_S, nl)[i];
         pa(I, q, PA_ALPHA, nl)[i] = sc * sc * tot[q];
         if (i >= 2) I.ps[q].itx = i - 1;
       }
+      __threadfence();
     }
     return;
   }
-  // PH_UPDATE: beta_{i+1}, s_{i+1}; then iteration i+1's top: breakdown test
-  // and the estimate with T(1:i), beta_{i+1}
-  __shared__ int est_q[kBatchMaxRhs];
-  __shared__ int nest;
+  // PH_UPDATE: beta_{i+1}, s_{i+1}; then iteration i+1's top: the breakdown
+  // test, and the pairs whose estimate of an earlier step has converged
   if (I.N > 0) {
     finalize_quad<R>(I, i, B, tot);
     return;
   }
-  if (threadIdx.x == 0) {
-    nest = 0;
-    for (int q = 0; q < R; ++q) {
-      PairState& P = I.ps[q];
-      if (P.done) continue;
+  if (threadIdx.x < R) {  // a thread per pair: the square root and the division of all pairs at once
+    const int q = threadIdx.x;
+    PairState& P = I.ps[q];
+    if (!P.done) {
       const double sc = pa(I, q, PA_S, nl)[i];
       const double wn = sqrt(tot[q]);
       const double beta = sc * wn;
       pa(I, q, PA_BETA, nl)[i + 1] = beta;
-      pa(I, q, PA_S, nl)[i + 1] = 1.0 / ldexp(wn, ilog2_normal(sc));
-      if (i + 1 > nl) { P.done = 1; continue; }
+      const double sn = 1.0 / ldexp(wn, ilog2_normal(sc));
+      pa(I, q, PA_S, nl)[i + 1] = sn;
+      pa(I, q, PA_C2, nl)[i + 1] = beta * sc / sn;
       P.itx = i;
-      if (fabs(beta) < 1e-16) { P.done = 1; continue; }  // psfun_d_lanczos.f90:225-230
-      if (B.istop == 1) est_q[nest++] = q;
-      else if (i + 1 == nl) P.done = 1;
+      if (fabs(beta) < 1e-16 || i + 1 >= nl) P.done = 1;  // psfun_d_lanczos.f90:225-230; the last iteration
+      if (*(volatile int*)&I.conv[q] != kConvNone) P.done = 1;
     }
-  }
-  __syncthreads();
-  if (nest > 0) {
-    // yk = exp(t T(1:i)) e1 for the pairs still running
-    unsigned mask = 0u;
-    for (int e = 0; e < nest; ++e) mask |= 1u << est_q[e];
-    if (!block_fT(I, nl, i, mask)) {
-      if (threadIdx.x == 0)
-        for (int e = 0; e < nest; ++e) { I.ps[est_q[e]].done = 1; I.ps[est_q[e]].info = PSFUN_ERR_FROM_SUBROUTINE_NON; }
-    } else if (threadIdx.x == 0) {
-      for (int e = 0; e < nest; ++e) {
-        const int q = est_q[e];
-        PairState& P = I.ps[q];
-        const double* yk = pa(I, q, PA_YK, nl);
-        double ss = 0.0;
-        for (int j = 0; j < i; ++j) ss += yk[j] * yk[j];
-        const double errnum = P.beta0 * fabs(I.t * pa(I, q, PA_BETA, nl)[i + 1]) * fabs(yk[i - 1]);
-        const double errden = sqrt(ss);
-        P.errnum = errnum;
-        P.errden = errden;
-        pa(I, q, PA_RS, nl)[i + 1] = errnum / errden;
-        if (errnum / errden < B.eps) {
-          P.done = 1;
-          P.conv = 1;
-          P.yk_len = i;
-          // keep the converged coefficients apart from later estimates
-          double* cf = pa(I, q, PA_COEF, nl);
-          for (int j = 0; j < i; ++j) cf[j] = yk[j];
-        } else if (i + 1 == nl) {
-          P.done = 1;  // loop ends after iteration nl
-        }
-      }
-    }
+    __threadfence();
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -722,6 +743,104 @@ PSF_DEVINL void finalize(const BInst& I, int ph, int i, const BatchArgs& B, doub
     for (int q = 0; q < R; ++q) live += !I.ps[q].done;
     if (live == 0 && I.cnt[1] != 0) atomicSub(B.active, 1u);
     I.cnt[1] = live;
+    st_release_gpu(reinterpret_cast<int*>(&I.cnt[2]), (int)((unsigned)i | (live == 0 ? kPubEnd : 0u)));
+  }
+}
+
+// The estimate of iteration i + 1 (T(1:i), beta_{i+1}) for the running pairs
+// of an instance, by one warp: the 7 R pole solves on a lane each, then
+// lane q the sums of pair q.
+template <int R>
+PSF_DEVINL void warp_estimate(const BInst& I, int i, const BatchArgs& B, zc* scr) {
+  static_assert(7 * R <= 32, "one pole per lane");
+  const int nl = B.nl, lane = threadIdx.x & 31;
+  const size_t stride = (size_t)(nl + 2);
+  double* yk = reinterpret_cast<double*>(scr + (size_t)R * 7 * 5 * stride);  // R rows of 2 ((nl + 3) / 2)
+  const size_t ldy = 2 * (size_t)((nl + 3) / 2);
+  const int q = lane / 7, p = lane - 7 * q;
+  bool run = false;
+  if (q < R) {
+    const volatile PairState& P = I.ps[q];
+    const double bn = pa(I, q, PA_BETA, nl)[i + 1];
+    run = P.beta0 != 0.0 && !(fabs(bn) < 1e-16) && i + 1 <= nl && *(volatile int*)&I.conv[q] > 2 * i;
+  }
+  // decided once per pair (its first lane), as conv may change meanwhile
+  const unsigned rb = __ballot_sync(0xffffffffu, run);
+  run = q < R && ((rb >> (7 * q)) & 1u);
+  if (rb == 0u) return;
+  int bad = 0;
+  if (run) {
+    zc* base = scr + (size_t)lane * 5 * stride;
+    cram_pole_tridiag(i, I.t, pa(I, q, PA_ALPHA, nl), pa(I, q, PA_BETA, nl), p, base + stride, base, &bad);
+  }
+  const bool any_bad = __any_sync(0xffffffffu, bad);  // ends the pairs that run, as in block_fT
+  if (any_bad) {
+    if (run && p == 0) atomicMin(&I.conv[q], 2 * i + 1);
+    return;
+  }
+  __syncwarp();
+  for (int task = lane; task < R * i; task += 32) {
+    const int qq = task / i, j = task - qq * i;
+    double acc = (j == 0) ? kCramAlpha0 : 0.0;
+    for (int pp = 0; pp < 7; ++pp)
+      acc = acc + cuCreal(zmul(zmk(kCramAlpha[pp][0], kCramAlpha[pp][1]), scr[((size_t)qq * 7 + pp) * 5 * stride + j]));
+    yk[qq * ldy + j] = acc;
+  }
+  __syncwarp();
+  if (run && p == 0) {
+    double ss = 0.0;
+    for (int j = 0; j < i; ++j) ss += yk[q * ldy + j] * yk[q * ldy + j];
+    const double errnum = I.ps[q].beta0 * fabs(I.t * pa(I, q, PA_BETA, nl)[i + 1]) * fabs(yk[q * ldy + i - 1]);
+    const double errden = sqrt(ss);
+    double* e = I.est + (size_t)q * 2 * stride + 2 * i;
+    e[0] = errnum;
+    e[1] = errden;
+    const double ratio = errnum / errden;
+    pa(I, q, PA_RS, nl)[i + 1] = ratio;
+    if (ratio < B.eps) atomicMin(&I.conv[q], 2 * i);
+  }
+  __syncwarp();
+}
+
+// A monitor block: estimates (instance k, step i), counted with the instances
+// fastest, go to the monitor warps of the grid in turn; each waits (bounded)
+// until its step is published, or leaves it out when the instance has ended
+// before.  The steps do not wait for the estimates: a pair whose estimate
+// converges meanwhile stops a step or two later, which changes nothing that
+// its result uses (later basis slots and entries of T), and the first
+// converged iteration is the one taken, as in the serial order.  On the
+// finalising block an estimate of order 17 costs ~100 us between two grid
+// barriers, with every other SM waiting; 24 uneven graphs (2-65 thousand
+// rows, 4 right-hand sides): 7.60 -> 4.87 ms with the cheaper
+// phases below, 7.0 by the monitors alone.
+template <int R>
+PSF_DEVINL void batch_monitor(const BatchArgs& B, int mb) {
+  const int warp = threadIdx.x >> 5;
+  if (warp >= kBatchMonWarps) return;
+  const int w = mb * kBatchMonWarps + warp, nw = B.monitors * kBatchMonWarps;
+  zc* scr = B.mon_scr + (size_t)w * batch_mon_zc(R, B.nl);
+  const long long total = (long long)B.count * (B.nl - 1);
+  for (long long task = w; task < total; task += nw) {
+    const int i = 1 + (int)(task / B.count);
+    const BInst& I = B.inst[task % B.count];
+    unsigned p = ld_acquire_gpu(&I.cnt[2]);
+    if ((p & ~kPubEnd) < (unsigned)i && !(p & kPubEnd)) {
+      const unsigned long long t0 = globaltimer_ns();
+      do {
+        __nanosleep(200);
+        if (*(volatile int*)B.err != 0) return;
+        if (globaltimer_ns() - t0 > kWaitLimitNs) {
+          atomicOr(B.err, DEVERR_TIMEOUT);
+          return;
+        }
+        p = ld_acquire_gpu(&I.cnt[2]);
+      } while ((p & ~kPubEnd) < (unsigned)i && !(p & kPubEnd));
+    }
+    __threadfence();
+    __syncwarp();
+    // (lanes may have read different values: the decision is the lowest)
+    const unsigned pub = __reduce_min_sync(0xffffffffu, p & ~kPubEnd);
+    if (pub >= (unsigned)i) warp_estimate<R>(I, i, B, scr);
   }
 }
 
@@ -734,34 +853,53 @@ PSF_DEVINL void final_pairs(const BInst& I, const BatchArgs& B, double* red) {
   }
   const int nl = B.nl;
   __shared__ int mq[kBatchMaxRhs];
-  __shared__ int need;
-  if (threadIdx.x == 0) {
-    need = 0;
-    for (int q = 0; q < R; ++q) {
-      PairState& P = I.ps[q];
-      mq[q] = 0;
-      if (P.info || P.beta0 == 0.0) continue;
-      if (!P.conv) {
-        const int m = P.itx - 1;
-        if (m < 1) { P.info = PSFUN_ERR_FROM_SUBROUTINE_NON; continue; }
-        mq[q] = m;
-        need = max(need, m);
+  if (threadIdx.x < R) {
+    const int q = threadIdx.x;
+    PairState& P = I.ps[q];
+    const int cv = I.conv[q];
+    mq[q] = 0;
+    if (!P.info && P.beta0 != 0.0) {
+      // the last iteration that had an estimate: none at a breakdown
+      int last = P.itx;
+      if (fabs(pa(I, q, PA_BETA, nl)[P.itx + 1]) < 1e-16) --last;
+      if (cv != kConvNone) {
+        P.itx = cv >> 1;
+        last = P.itx - (cv & 1);
+        if (cv & 1) {
+          P.info = PSFUN_ERR_FROM_SUBROUTINE_NON;
+        } else {
+          P.conv = 1;
+          mq[q] = P.itx;
+        }
+      } else {
+        mq[q] = P.itx - 1;
+        if (mq[q] < 1) P.info = PSFUN_ERR_FROM_SUBROUTINE_NON;
+      }
+      if (B.istop == 1 && last >= 1) {
+        const double* e = I.est + (size_t)q * 2 * (nl + 2) + 2 * last;
+        P.errnum = e[0];
+        P.errden = e[1];
       }
     }
   }
   __syncthreads();
-  // pairs that did not converge: f(T(1:itx-1)); pairs share the dimension only
-  // when equal, so evaluate per distinct m
+  // f(T(1:m)), m the converged iteration or itx-1; one evaluation for the
+  // pairs that share m
   for (int q = 0; q < R; ++q) {
     const int m = mq[q];
-    if (m == 0) continue;
-    if (!block_fT(I, nl, m, 1u << q)) {
-      if (threadIdx.x == 0) I.ps[q].info = PSFUN_ERR_FROM_SUBROUTINE_NON;
-      continue;
-    }
-    if (threadIdx.x == 0) {
-      for (int j = 0; j < m; ++j) pa(I, q, PA_COEF, nl)[j] = pa(I, q, PA_YK, nl)[j];
-      I.ps[q].yk_len = m;
+    if (m < 1) continue;
+    unsigned mask = 0u;
+    for (int o = 0; o < R; ++o) mask |= (mq[o] == m) ? 1u << o : 0u;
+    if (mask & ((1u << q) - 1u)) continue;  // evaluated with an earlier pair
+    const bool ok = block_fT(I, nl, m, mask);
+    if (threadIdx.x < R && ((mask >> threadIdx.x) & 1u)) {
+      const int o = threadIdx.x;
+      if (!ok) {
+        I.ps[o].info = PSFUN_ERR_FROM_SUBROUTINE_NON;
+      } else {
+        for (int j = 0; j < m; ++j) pa(I, o, PA_COEF, nl)[j] = pa(I, o, PA_YK, nl)[j];
+        I.ps[o].yk_len = m;
+      }
     }
     __syncthreads();
   }
@@ -787,36 +925,6 @@ PSF_DEVINL bool tile_staged(const BInst& I, int lt) {
   return ti.k1 - ti.k0 <= kTileNnz;
 }
 
-// Sums of the R per-thread values over the block, for thread 0: each warp's
-// butterfly, then the warps in order.  red holds 16 * R doubles; it is
-// rewritten only after the caller's next block barrier.
-template <int R>
-PSF_DEVINL void block_sum_R(const double* acc, double* red, double* out) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  double v[R];
-#pragma unroll
-  for (int q = 0; q < R; ++q) v[q] = acc[q];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-    for (int q = 0; q < R; ++q) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
-  }
-  if (lane == 0) {
-#pragma unroll
-    for (int q = 0; q < R; ++q) red[wid * R + q] = v[q];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nw = blockDim.x >> 5;
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      double t = 0.0;
-      for (int w = 0; w < nw; ++w) t += red[w * R + q];
-      out[q] = t;
-    }
-  }
-}
-
 // The update phase over rows [rb, re) of instance I (whole runs of tiles):
 // W_{i+1} = 2^k (u - alpha W_i - c W_{i-1}) for the live pairs, the norms'
 // partial sums in accR; several rows per thread in flight.
@@ -832,7 +940,7 @@ PSF_DEVINL void update_rows(const BInst& I, int i, int rb, int re, const BatchAr
   for (int q = 0; q < R; ++q) {
     const double sc = pa(I, q, PA_S, B.nl)[i];
     c1[q] = pa(I, q, PA_ALPHA, B.nl)[i];
-    c2[q] = (i >= 2) ? pa(I, q, PA_BETA, B.nl)[i] * pa(I, q, PA_S, B.nl)[i - 1] / sc : 0.0;
+    c2[q] = pa(I, q, PA_C2, B.nl)[i];
     k2[q] = ilog2_normal(sc);
     live[q] = !I.ps[q].done;
   }
@@ -877,116 +985,125 @@ PSF_DEVINL void update_rows(const BInst& I, int i, int rb, int re, const BatchAr
 
 constexpr int kBatchChunkMax = 16;  // queue tiles taken per grab, at most (B.chunk)
 
-// One phase over the global tile queue.  A block takes B.chunk
-// consecutive tiles per grab; in the SpMM phase the next tile of the chunk is
-// staged by TMA into the other buffer while the current one is computed.
-// The tiles of each instance in the chunk are counted with one atomic; the
-// block that completes an instance finalises it.
+// What a block has taken from the queue: tiles [g0, g0 + B.chunk), g0 < 0
+// after a device error.
+struct Grab {
+  int g0;
+  int inst[kBatchChunkMax];
+  unsigned char skip[kBatchChunkMax], staged[kBatchChunkMax];
+};
+
+// One phase over the global tile queue.  A block takes B.chunk consecutive
+// tiles per grab.  Its last warp (the one without rows in a full SpMM tile)
+// takes the next grab while the current one is computed, and in the SpMM phase
+// stages the next tile, of this grab or the next, into the other buffer.
+// The tiles of each instance in the grab are counted with one atomic; the
+// block that completes an instance finalises it.  Tiles of ended instances
+// are passed over.
 template <int R>
 PSF_DEVINL bool run_phase(const BatchArgs& B, int ph, int i, unsigned* qctr, SpmvSmem& sm) {
-  __shared__ int g0_sh, last_sh;
-  __shared__ int inst_sh[kBatchChunkMax];
-  __shared__ unsigned char skip_sh[kBatchChunkMax], staged_sh[kBatchChunkMax];
+  __shared__ int last_sh;
+  __shared__ Grab grabs[2];
   __shared__ double redR[16 * kBatchMaxRhs];
-  for (;;) {
-    if (threadIdx.x < 32) {
-      // -1 drains the queue after a device error; decided once per block.
-      // Lanes 0..B.chunk-1 look up one tile each, in parallel.
-      int g0 = 0;
-      if (threadIdx.x == 0) g0 = (*(volatile int*)B.err != 0) ? -1 : (int)atomicAdd(qctr, (unsigned)B.chunk);
-      g0 = __shfl_sync(0xffffffffu, g0, 0);
-      const int c = threadIdx.x;
-      if (c == 0) g0_sh = g0;
-      if (g0 >= 0 && c < B.chunk && g0 + c < B.total_tiles) {
-        const int g = g0 + c;
-        const int k = find_inst(B, g);
-        inst_sh[c] = k;
-        const BInst& I = B.inst[k];
-        const bool skip = (ph != PH_INIT && ph != PH_RECOMB) && (*(volatile unsigned*)&I.cnt[1] == 0u);
-        skip_sh[c] = skip;
-        const bool st = (ph == PH_SPMM && !skip && tile_staged(I, g - I.tile_begin));
-        staged_sh[c] = st;
-        if (c == 0 && st) spmv_issue(I.A, tile_info(I.A, g - I.tile_begin), sm, 0);
-      }
+  const int lane = threadIdx.x & 31;
+  const bool fetcher = (threadIdx.x >> 5) == (blockDim.x >> 5) - 1;
+  // by one warp; lanes 0..B.chunk-1 look up one tile each, in parallel
+  auto grab = [&](Grab& gr) {
+    int g0 = 0;
+    if (lane == 0) g0 = (*(volatile int*)B.err != 0) ? -1 : (int)atomicAdd(qctr, (unsigned)B.chunk);
+    g0 = __shfl_sync(0xffffffffu, g0, 0);
+    if (lane == 0) gr.g0 = g0;
+    if (g0 >= 0 && lane < B.chunk && g0 + lane < B.total_tiles) {
+      const int g = g0 + lane;
+      const int k = find_inst(B, g);
+      gr.inst[lane] = k;
+      const BInst& I = B.inst[k];
+      const bool skip = (ph != PH_INIT && ph != PH_RECOMB) && (*(volatile unsigned*)&I.cnt[1] == 0u);
+      gr.skip[lane] = skip;
+      gr.staged[lane] = (ph == PH_SPMM && !skip && tile_staged(I, g - I.tile_begin));
     }
-    __syncthreads();
-    const int g0 = g0_sh;
+    __syncwarp();
+  };
+  auto stage = [&](const Grab& gr, int c, int buf) {
+    if (lane == 0 && gr.g0 >= 0 && gr.g0 + c < B.total_tiles && gr.staged[c]) {
+      const BInst& I = B.inst[gr.inst[c]];
+      spmv_issue(I.A, tile_info(I.A, gr.g0 + c - I.tile_begin), sm, buf);
+    }
+  };
+  int cur = 0, buf = 0;
+  if (fetcher) {
+    grab(grabs[0]);
+    if (ph == PH_SPMM) stage(grabs[0], 0, 0);
+  }
+  __syncthreads();
+  for (;; cur ^= 1) {
+    const Grab& gr = grabs[cur];
+    const int g0 = gr.g0;
     if (g0 < 0 || g0 >= B.total_tiles) break;
     const int nc = min(B.total_tiles, g0 + B.chunk) - g0;
-    // runs of consecutive tiles of one instance (chunk boundaries are fixed
+    if (ph != PH_SPMM && fetcher) grab(grabs[cur ^ 1]);
+    // runs of consecutive tiles of one instance (grab boundaries are fixed
     // multiples of B.chunk, so the runs and their partial slots are the
-    // same whichever block takes the chunk)
+    // same whichever block takes the grab)
     for (int c = 0; c < nc;) {
-      const int k = inst_sh[c];
+      const int k = gr.inst[c];
       int ce = c + 1;
-      while (ce < nc && inst_sh[ce] == k) ++ce;
+      while (ce < nc && gr.inst[ce] == k) ++ce;
       const BInst& I = B.inst[k];
-      const bool skip = skip_sh[c] != 0;
-      const size_t pslot = (size_t)((ph == PH_UPDATE) ? 1 : 0) * I.ntiles;
+      const bool skip = gr.skip[c] != 0;
+      const int lt0 = g0 + c - I.tile_begin, lt1 = g0 + ce - I.tile_begin;
+      double accR[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) accR[q] = 0.0;
       if (ph == PH_UPDATE) {
-        // the whole run at once; its partial in the slot of its first tile
-        const int lt0 = g0 + c - I.tile_begin, lt1 = g0 + ce - I.tile_begin;
-        double accR[R];
-#pragma unroll
-        for (int q = 0; q < R; ++q) accR[q] = 0.0;
+        // the whole run at once
         if (!skip) update_rows<R>(I, i, I.A.tile_desc[lt0].x, I.A.tile_desc[lt1].x, B, accR);
-        double tot[R];
-        block_sum_R<R>(accR, redR, tot);
-        if (threadIdx.x == 0) {
-          for (int lt = lt0; lt < lt1; ++lt) {
-            double* part = I.part + (pslot + lt) * R;
-#pragma unroll
-            for (int q = 0; q < R; ++q) part[q] = (lt == lt0) ? tot[q] : 0.0;
-          }
-        }
       } else {
-        // tile by tile (the SpMM stages each tile, double-buffered), the
-        // run's partial summed once, in the slot of its first tile
-        double accR[R];
-#pragma unroll
-        for (int q = 0; q < R; ++q) accR[q] = 0.0;
+        // tile by tile (the SpMM stages each tile, double-buffered)
         for (int cc = c; cc < ce; ++cc) {
-          const int g = g0 + cc, b = cc & 1;
-          const int lt = g - I.tile_begin;
-          if (threadIdx.x == 0 && cc + 1 < nc && staged_sh[cc + 1]) {
-            const BInst& In = B.inst[inst_sh[cc + 1]];
-            spmv_issue(In.A, tile_info(In.A, g + 1 - In.tile_begin), sm, b ^ 1);
-          }
-          if (!skip) tile_work<R>(I, ph, i, lt, B, sm, accR, b);
-          __syncthreads();  // the tile's buffer is free for the next prefetch
-        }
-        if (ph != PH_RECOMB) {
-          const int lt0 = g0 + c - I.tile_begin, lt1 = g0 + ce - I.tile_begin;
-          double tot[R];
-          block_sum_R<R>(accR, redR, tot);
-          if (threadIdx.x == 0) {
-            for (int lt = lt0; lt < lt1; ++lt) {
-              double* part = I.part + (pslot + lt) * R;
-#pragma unroll
-              for (int q = 0; q < R; ++q) part[q] = (lt == lt0) ? tot[q] : 0.0;
+          if (ph == PH_SPMM && fetcher) {
+            if (cc + 1 < nc) {
+              stage(gr, cc + 1, buf ^ 1);
+            } else {
+              grab(grabs[cur ^ 1]);
+              stage(grabs[cur ^ 1], 0, buf ^ 1);
             }
+          }
+          if (!skip) tile_work<R>(I, ph, i, g0 + cc - I.tile_begin, B, sm, accR, buf);
+          if (ph == PH_SPMM) {
+            buf ^= 1;
+            __syncthreads();  // the tile's buffer is free for the next prefetch
           }
         }
       }
-      if (ph != PH_RECOMB) {
-        // the run's tiles are counted at once; the block completing the
-        // instance finalises it
-        if (threadIdx.x == 0) {
-          __threadfence();
-          last_sh = (atomicAdd(&I.cnt[0], (unsigned)(ce - c)) + (unsigned)(ce - c) == (unsigned)I.ntiles);
+      if (ph != PH_RECOMB && !skip) {
+        // the run's partial, in the slot of its first tile; the run's tiles
+        // are counted at once, and the block completing the instance
+        // finalises it
+        double* part = I.part + ((size_t)((ph == PH_UPDATE) ? 1 : 0) * I.ntiles + lt0) * R;
+        block_sum_R<R>(accR, redR, part);
+        if (threadIdx.x < 32) {
+          for (int e = R + lane; e < (lt1 - lt0) * R; e += 32) part[e] = 0.0;
+          __syncwarp();
+          if (lane == 0) {
+            __threadfence();
+            last_sh = (atomicAdd(&I.cnt[0], (unsigned)(ce - c)) + (unsigned)(ce - c) == (unsigned)I.ntiles);
+          }
         }
         __syncthreads();
         if (last_sh) {
           __threadfence();
           if (threadIdx.x == 0) I.cnt[0] = 0u;
-          if (!skip) finalize<R>(I, ph, i, B, sm.red);
+          finalize<R>(I, ph, i, B, redR);
           __threadfence();
+          __syncthreads();  // redR and last_sh are free
         }
       }
-      __syncthreads();
       c = ce;
     }
+    __syncthreads();  // the next grab is in place
   }
+  __syncthreads();  // grabs is free
   return true;
 }
 
@@ -994,22 +1111,31 @@ template <int R>
 __global__ void __launch_bounds__(kBatchThreads, 1) k_batch(BatchArgs B) {
   PSF_SPMV_SMEM();
   spmv_smem_init(sm);
-  int ph_idx = 0;
-  run_phase<R>(B, PH_INIT, 0, &B.queue[ph_idx++], sm);
-  if (!grid_barrier(&B.bar[0], &B.bar[1], B.err)) return;
-  __shared__ unsigned act;
-  for (int i = 1; i <= B.nl; ++i) {
-    if (threadIdx.x == 0) act = *(volatile unsigned*)B.active;
-    __syncthreads();
-    if (act == 0u) break;  // block-uniform; identical in every block after the barrier
-    run_phase<R>(B, PH_SPMM, i, &B.queue[ph_idx++], sm);
-    if (!grid_barrier(&B.bar[0], &B.bar[1], B.err)) return;
-    run_phase<R>(B, PH_UPDATE, i, &B.queue[ph_idx++], sm);
-    if (!grid_barrier(&B.bar[0], &B.bar[1], B.err)) return;
+  const unsigned G = gridDim.x - B.monitors;
+  unsigned nb = 0;
+  auto gsync = [&]() { return grid_sync_to(&B.bar[0], (++nb) * G, B.err); };  // the blocks that run the steps
+  if (blockIdx.x >= G) {
+    batch_monitor<R>(B, blockIdx.x - G);
+  } else {
+    int ph_idx = 0;
+    run_phase<R>(B, PH_INIT, 0, &B.queue[ph_idx++], sm);
+    if (!gsync()) return;
+    __shared__ unsigned act;
+    for (int i = 1; i <= B.nl; ++i) {
+      if (threadIdx.x == 0) act = *(volatile unsigned*)B.active;
+      __syncthreads();
+      if (act == 0u) break;  // block-uniform; identical in every block after the barrier
+      run_phase<R>(B, PH_SPMM, i, &B.queue[ph_idx++], sm);
+      if (!gsync()) return;
+      run_phase<R>(B, PH_UPDATE, i, &B.queue[ph_idx++], sm);
+      if (!gsync()) return;
+    }
   }
-  // final f per instance (CTA k handles instances k, k+G, ...)
+  // the steps and every estimate are done: final f per instance (CTA k
+  // handles instances k, k+G, ...), on all blocks
+  if (!grid_sync_to(&B.bar[1], gridDim.x, B.err)) return;
   for (int k = blockIdx.x; k < B.count; k += gridDim.x) final_pairs<R>(B.inst[k], B, sm.red);
-  if (!grid_barrier(&B.bar[0], &B.bar[1], B.err)) return;
+  if (!grid_sync_to(&B.bar[1], 2 * gridDim.x, B.err)) return;
   run_phase<R>(B, PH_RECOMB, 0, &B.queue[2 * B.nl + 2], sm);
 }
 
@@ -1116,13 +1242,14 @@ static int batch_launch(BatchArgs& B, std::vector<BInst>& hinst, BInst* dinst, c
   int per = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch<R>, kBatchThreads, kSpmvSmemBytes);
   if (per < 1) per = 1;
-  int G = sm_count() * per;
+  int G = std::max(1, sm_count() * per - B.monitors);
   if (G > B.total_tiles) G = std::max(1, B.total_tiles);
   // about four grabs per block and phase, at most kBatchChunkMax tiles each:
   // larger grabs amortise the queue and per-run costs, smaller ones balance
   B.chunk = std::max(1, std::min(kBatchChunkMax, B.total_tiles / (4 * G)));
   void* args[] = {(void*)&B};
-  PSF_CUDA(cudaLaunchCooperativeKernel((void*)k_batch<R>, dim3(G), dim3(kBatchThreads), args, kSpmvSmemBytes, s));
+  PSF_CUDA(cudaLaunchCooperativeKernel((void*)k_batch<R>, dim3(G + B.monitors), dim3(kBatchThreads), args,
+                                       kSpmvSmemBytes, s));
   count_launch();
   return PSFUN_SUCCESS;
 }
@@ -1157,7 +1284,8 @@ static int batch_run(DevBuf* wsbuf, int keeplast, int mapping, int count, const 
     off += (doubles + 31) & ~(size_t)31;
     return o;
   };
-  std::vector<size_t> oV(count), oU(count), oS(count), oP(count), oC(count), oPS(count), oCnt(count), oQ2(count);
+  std::vector<size_t> oV(count), oU(count), oS(count), oP(count), oC(count), oPS(count), oCnt(count), oQ2(count),
+      oE(count);
   for (int k = 0; k < count; ++k) {
     psfun_csr* a = items[k].a;
     BInst& I = hinst[k];
@@ -1180,7 +1308,15 @@ static int batch_run(DevBuf* wsbuf, int keeplast, int mapping, int count, const 
     oQ2[k] = carve(items[k].N > 0 ? (size_t)4 * items[k].N + (size_t)R * 4 * items[k].N : 0);
     oPS[k] = carve((sizeof(PairState) * R + 7) / 8);
     oCnt[k] = carve(2);
+    oE[k] = carve(items[k].N > 0 ? 0 : (size_t)R * 2 * (nl + 2));
   }
+  // Monitor blocks: three warps per instance cover a step (>= 12 us) for
+  // estimates of up to ~36 us, at most a tenth of the SMs.
+  const bool estimates = istop == 1 && items[0].N == 0;
+  const int monitors =
+      estimates ? std::max(1, std::min(sm_count() / 10, (3 * count + kBatchMonWarps - 1) / kBatchMonWarps)) : 0;
+  const size_t oMon = carve((size_t)monitors * kBatchMonWarps * batch_mon_zc(R, nl) * 2);
+  const size_t oConv = carve(((size_t)count * R + 1) / 2);
   const size_t oInst = carve((sizeof(BInst) * count + 7) / 8);
   const size_t oQ = carve(2 * (size_t)nl + 8);
   const size_t oMisc = carve(8);
@@ -1193,6 +1329,7 @@ static int batch_run(DevBuf* wsbuf, int keeplast, int mapping, int count, const 
     PSF_CUDA(cudaMemsetAsync(base + oS[k], 0, sizeof(double) * (oP[k] - oS[k]), s));
     PSF_CUDA(cudaMemsetAsync(base + oPS[k], 0, sizeof(double) * (oInst > oPS[k] ? (oCnt[k] + 2 - oPS[k]) : 0), s));
   }
+  PSF_CUDA(cudaMemsetAsync(base + oConv, 0x7f, sizeof(int) * (size_t)count * R, s));
   PSF_CUDA(cudaMemsetAsync(base + oQ, 0, sizeof(double) * (oMisc + 8 - oQ), s));
   for (int k = 0; k < count; ++k) {
     BInst& I = hinst[k];
@@ -1203,6 +1340,8 @@ static int batch_run(DevBuf* wsbuf, int keeplast, int mapping, int count, const 
     I.cram = base + oC[k];
     I.ps = reinterpret_cast<PairState*>(base + oPS[k]);
     I.cnt = reinterpret_cast<unsigned*>(base + oCnt[k]);
+    I.conv = reinterpret_cast<int*>(base + oConv) + (size_t)k * R;
+    I.est = base + oE[k];
     I.N = items[k].N;
     if (I.N > 0) {  // shifts and weights, then the pairs' recurrence state
       double* q = base + oQ2[k];
@@ -1236,6 +1375,8 @@ static int batch_run(DevBuf* wsbuf, int keeplast, int mapping, int count, const 
   B.err = reinterpret_cast<int*>(misc + 2);
   B.active = misc + 3;
   B.tile_inst = dti;
+  B.monitors = monitors;
+  B.mon_scr = reinterpret_cast<zc*>(base + oMon);
   const unsigned active = (unsigned)count;
   PSF_CUDA(cudaMemcpyAsync(B.active, &active, sizeof active, cudaMemcpyHostToDevice, s));
   int rc;
