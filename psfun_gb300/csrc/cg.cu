@@ -225,7 +225,9 @@ __global__ void k_diag_inv(int64_t n, const double* d, double* out) {
 //   x += alpha p, r -= alpha q, z = D r, partial r.z and the norms of the
 //   stopping rule                                      -> barrier -> stop, beta
 // Thread 0 of every block forms the same scalars from the per-block partials
-// in the same order; block 0 records them in the control block.  The kernel
+// in the same order; block 0 records them in the control block.  The maxima of the stopping rule are taken as integers
+// of the values' bits (two FP64 maxima per row would be a third of the update's
+// time on the FP64 pipe).  @@CG@@  The kernel
 // returns when the stopping rule holds, itx reaches itmax, or a breakdown
 // (sigma = 0 or rho_old = 0) asks the host to restart.
 // ---------------------------------------------------------------------------
@@ -247,7 +249,7 @@ __global__ void __launch_bounds__(kSpmvThreads) k_cg_persist(CgState st, CsrDev 
   if (threadIdx.x == kConsumerWarps * 32) {
     if (!pipe_produce(A, t0, t0 + min(kLzStages, t1 - t0), sm, pc.issued, stream)) atomicOr(&c->err, DEVERR_TIMEOUT);
   }
-  double* part = st.part;  // [5][G]
+  double* part = st.part;  // [4][G]: p.q, r.z, the norms of r and x
   unsigned nb = 0;
   unsigned passes = 0;  // SpMV passes completed (each consumes t1 - t0 tiles)
   auto drain = [&]() { pipe_drain(sm, pc, passes * (unsigned)(t1 - t0)); };
@@ -262,15 +264,14 @@ __global__ void __launch_bounds__(kSpmvThreads) k_cg_persist(CgState st, CsrDev 
       return;
     }
     ++passes;
-    if (!bj) block_sum_store_512(epi.acc, sm.vals, sm.red, &part[bid]);
-  }
-  if (!gsync()) { drain(); return; }
-  if constexpr (BJ) {  // z = M^{-1} r once r is complete, then rho = r.z
-    block_sum_store_512(bjac_solve_blocks(st, rb, re), sm.vals, sm.red, &part[bid]);
+    double S = epi.acc;
+    if constexpr (BJ) {  // z = M^{-1} r once r is complete, then rho = r.z
+      if (!gsync()) { drain(); return; }
+      S = bjac_solve_blocks(st, rb, re);
+    }
+    block_sum_store_512(S, sm.vals, sm.red, &part[G + bid]);
     if (!gsync()) { drain(); return; }
-  }
-  {
-    const double S = partials_sum_to0(part, G, sm.red);
+    partials_reduce_to0(part + G, G, 1, 1, G, sm.vals, &S);
     if (threadIdx.x == 0) {
       sm.scal[0] = S;
       if (bid == 0) {
@@ -312,18 +313,17 @@ __global__ void __launch_bounds__(kSpmvThreads) k_cg_persist(CgState st, CsrDev 
     if (!gsync()) { drain(); return; }
     // ---- q = eta A p + zeta p ; sigma = p.q ; alpha = rho / sigma (:302-310)
     {
-      EpiShiftDot epi{st.eta, st.zeta, st.p, st.q, 0.0};
+      EpiShiftDot epi{st.eta, st.zeta, st.eta == 1.0, st.p, st.q, 0.0};
       if (__syncthreads_or(!pipe_spmv(A, st.p, t0, t1, sm, epi, &c->err, pc, true, stream))) {
         drain();
         return;
       }
       ++passes;
-      block_sum_store_512(epi.acc, sm.vals, sm.red, &part[G + bid]);
-    }
-    if (!gsync()) { drain(); return; }
-    ++itx;
-    {
-      const double sigma = partials_sum_to0(part + G, G, sm.red);
+      double sigma = 0.0;
+      block_sum_store_512(epi.acc, sm.vals, sm.red, &part[bid]);
+      if (!gsync()) { drain(); return; }
+      partials_reduce_to0(part, G, 1, 1, G, sm.vals, &sigma);
+      ++itx;
       if (threadIdx.x == 0) {
         sm.scal[1] = (sigma == 0.0) ? 0.0 : rho / sigma;
         sm.scal[2] = (sigma == 0.0) ? 1.0 : 0.0;
@@ -348,7 +348,12 @@ __global__ void __launch_bounds__(kSpmvThreads) k_cg_persist(CgState st, CsrDev 
     if (sm.scal[2] != 0.0) { drain(); return; }
     const double alpha = sm.scal[1];
     // ---- x += alpha p ; r -= alpha q ; z = D r ; rho' = r.z ; norms (:320-333)
-    double a_rz = 0.0, a_r = 0.0, a_x = 0.0;
+    double a_rz = 0.0, a_r = 0.0;
+    long long m_r = 0, m_x = 0;  // bits of max |r|, max |x|
+    auto vmax = [](long long m, double v) {
+      const long long b = __double_as_longlong(v) & 0x7fffffffffffffffLL;
+      return (b > m && b <= 0x7ff0000000000000LL) ? b : m;  // NaN is passed over, as fmax does
+    };
     auto upd = [&](int r, double pv, double xo, double qv, double ro, double dv) {
       const double xv = fma(alpha, pv, xo);
       st.x[r] = xv;
@@ -360,8 +365,8 @@ __global__ void __launch_bounds__(kSpmvThreads) k_cg_persist(CgState st, CsrDev 
         a_rz = fma(rv, zv, a_rz);
       }
       if (st.istop == 1) {
-        a_r = fmax(a_r, fabs(rv));
-        a_x = fmax(a_x, fabs(xv));
+        m_r = vmax(m_r, rv);
+        m_x = vmax(m_x, xv);
       } else {
         a_r = fma(rv, rv, a_r);
       }
@@ -384,30 +389,39 @@ __global__ void __launch_bounds__(kSpmvThreads) k_cg_persist(CgState st, CsrDev 
       }
       for (; r < re; r += bd) upd(r, st.p[r], st.x[r], st.q[r], st.r[r], st.dinv ? st.dinv[r] : 1.0);
     }
-    if (!bj) block_sum_store_512(a_rz, sm.vals, sm.red, &part[2 * G + bid]);
     if (st.istop == 1) {
-      block_max_store_512(a_r, sm.vals, sm.red, &part[3 * G + bid]);
-      block_max_store_512(a_x, sm.vals, sm.red, &part[4 * G + bid]);
+      long long* sh = reinterpret_cast<long long*>(sm.vals) + 448;  // past what the other reductions use
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+      auto wmax = [](long long v) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+        return v;
+      };
+      m_r = wmax(m_r);
+      m_x = wmax(m_x);
+      if (lane == 0) {
+        sh[warp] = m_r;
+        sh[32 + warp] = m_x;
+      }
+      __syncthreads();
+      if (warp < 2) {
+        const long long v = wmax(lane < kSpmvThreads / 32 ? sh[32 * warp + lane] : 0);
+        if (lane == 0) part[(2 + warp) * G + bid] = __longlong_as_double(v);
+      }
+      __syncthreads();  // vals is free
     } else {
-      block_sum_store_512(a_r, sm.vals, sm.red, &part[3 * G + bid]);
+      block_sum_store_512(a_r, sm.vals, sm.red, &part[2 * G + bid]);
     }
-    if (!gsync()) { drain(); return; }
     if constexpr (BJ) {  // z = M^{-1} r once r is complete, then the partial r.z
-      __syncthreads();  // the norm reductions above are done with vals/red
-      block_sum_store_512(bjac_solve_blocks(st, rb, re), sm.vals, sm.red, &part[2 * G + bid]);
       if (!gsync()) { drain(); return; }
+      a_rz = bjac_solve_blocks(st, rb, re);
     }
     {
-      const double s_rz = partials_sum_to0(part + 2 * G, G, sm.red);
-      double s_r, s_x = 0.0;
-      __syncthreads();  // red is reused below
-      if (st.istop == 1) {
-        s_r = partials_max_to0(part + 3 * G, G, sm.red);
-        __syncthreads();
-        s_x = partials_max_to0(part + 4 * G, G, sm.red);
-      } else {
-        s_r = partials_sum_to0(part + 3 * G, G, sm.red);
-      }
+      double tot[3] = {0.0, 0.0, 0.0};
+      block_sum_store_512(a_rz, sm.vals, sm.red, &part[G + bid]);
+      if (!gsync()) { drain(); return; }
+      partials_reduce_to0(part + G, G, st.istop == 1 ? 3 : 2, st.istop == 1 ? 1 : 2, G, sm.vals, tot);
+      const double s_rz = tot[0], s_r = tot[1], s_x = tot[2];
       if (threadIdx.x == 0) {
         double errnum, errden;
         if (st.istop == 1) {

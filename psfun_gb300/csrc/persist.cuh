@@ -47,6 +47,47 @@ PSF_DEVINL void lz_smem_init(LzSmem& sm) {
   __syncthreads();
 }
 
+// The reductions k = 0 .. nk-1 of the blocks' partials p + k * ld (the first
+// `sums` of them sums, the others maxima of non-negative values; NaN is passed
+// over, as fmax does) over `count` <= 256 blocks, for thread 0 in tot[k]: all
+// fetched at once by different warps.  The order of partials_sum_to0.  scratch:
+// 8 nk doubles of shared memory.  All threads call it.
+PSF_DEVINL void partials_reduce_to0(const volatile double* p, int ld, int nk, int sums, int count, double* scratch,
+                                    double* tot) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int nch = (count + 31) >> 5;
+  for (int u = threadIdx.x >> 5; u < nk * nch; u += nw) {
+    const int k = u / nch, c = 32 * (u - k * nch) + lane;
+    double v = (c < count) ? p[(size_t)k * ld + c] : 0.0;
+    if (k < sums) {
+      v = warp_sum(v);
+    } else {
+      long long b = __double_as_longlong(v);
+      if (b > 0x7ff0000000000000LL) b = 0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
+      v = __longlong_as_double(b);
+    }
+    if (lane == 0) scratch[8 * k + (u - k * nch)] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < nk; ++k) {
+      double t[8];
+#pragma unroll
+      for (int w = 0; w < 8; ++w) t[w] = (w < nch) ? scratch[8 * k + w] : 0.0;
+      if (k < sums) {
+        tot[k] = ((t[0] + t[4]) + (t[2] + t[6])) + ((t[1] + t[5]) + (t[3] + t[7]));
+      } else {
+        long long m = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) m = max(m, __double_as_longlong(t[w]));
+        tot[k] = __longlong_as_double(m);
+      }
+    }
+  }
+}
+
 struct PipeCounters {
   unsigned issued;    // producer: tiles staged so far
   unsigned consumed;  // consumers: tiles consumed so far

@@ -275,28 +275,17 @@ struct EpiAxpby {
   }
 };
 
-// u = A*x with the partial dot sum_r u_r * x_r (Lanczos alpha; the scale of
-// x is folded into the scalars by the caller).
-struct EpiDot {
-  double* __restrict__ u;
-  const double* __restrict__ xown;
-  double acc;
-  PSF_DEVINL void operator()(int r, double s) {
-    u[r] = s;
-    acc = fma(s, xown[r], acc);
-  }
-};
-
 // q = eta*A*p + zeta*p with the partial dot sum_r p_r q_r (shifted CG,
 // psfun_dcg.F90:302-304).
 struct EpiShiftDot {
   double eta, zeta;
+  bool unit;  // eta == 1: the multiplication (exact) is left out
   const double* __restrict__ p;
   double* __restrict__ q;
   double acc;
   PSF_DEVINL void operator()(int r, double s) {
     const double pr = p[r];
-    const double v = fma(zeta, pr, eta * s);
+    const double v = fma(zeta, pr, unit ? s : eta * s);
     q[r] = v;
     acc = fma(pr, v, acc);
   }
