@@ -111,4 +111,94 @@ PSF_DEVINL long long ld_relaxed_s64(const long long* p) {
   return v;
 }
 
+// A still wider window for a squared norm that may be rounding noise of its
+// bound: p 2^(192-E) as four 48-bit limbs, lowest first; p >= 0.
+PSF_DEVINL bool fix192_limbs(double p, int E, long long (&w)[4]) {
+  const unsigned hi = (unsigned)__double2hiint(p), lo = (unsigned)__double2loint(p);
+  const int ex = (int)((hi >> 20) & 0x7ffu);
+  int pos = max(ex, 1) - (E + 883);  // p = m 2^(ex - 1075), the window's unit 2^(E - 192)
+  unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | (ex ? 0x100000u : 0u)) << 32) | lo;
+  const bool ok = pos <= 139 && ex != 0x7ff && (hi >> 31) == 0u;
+  m >>= min(max(-pos, 0), 63);
+  pos = min(max(pos, 0), 139);
+  const int q = pos >= 96 ? 2 : pos >= 48 ? 1 : 0;  // the limb that holds the lowest bit
+  const int ls = pos - 48 * q;
+  const long long l = (long long)((m << ls) & (unsigned long long)kFixMask48), h = (long long)(m >> (48 - ls));
+  w[0] = q == 0 ? l : 0;
+  w[1] = q == 0 ? h : q == 1 ? l : 0;
+  w[2] = q == 1 ? h : q == 2 ? l : 0;
+  w[3] = q == 2 ? h : 0;
+  return ok;
+}
+
+PSF_DEVINL double fix192_value(long long w3, long long w2, long long w1, long long w0, int E) {
+  w1 += w0 >> 48;
+  w0 &= kFixMask48;
+  w2 += w1 >> 48;
+  w1 &= kFixMask48;
+  w3 += w2 >> 48;
+  w2 &= kFixMask48;
+  const double c = 281474976710656.0;  // 2^48
+  const double v = fma(fma(fma((double)w3, c, (double)w2), c, (double)w1), c, (double)w0);
+  return scale_pow2(v, E - 192);
+}
+
+// ---------------------------------------------------------------------------
+// Grid sums whose words count their own arrivals.  Each block adds to every
+// limb's word, beside its signed 48-bit limb, 1 in the bits from 56 up; a
+// reader that finds G there has the sum.  The arrival and the value are one
+// word, so a reduction over the grid is one atomic and one L2 round trip past
+// the last block, where a counter barrier, the fetch of every block's partial
+// and their FP64 butterfly took 5500-6500 clocks (152 blocks; polling one slot
+// per block instead of one word per limb is no cure: 152 x 152 polls made the
+// same reduction 3000 clocks slower).  G <= 200; a block whose addend does not
+// fit the window marks the top limb, and the sum becomes NaN: the bound E
+// passed to it lies 3 bits above what the sum can reach, which keeps unmarked
+// top limbs below 2^46.
+// ---------------------------------------------------------------------------
+constexpr int kCountMaxBlocks = 200;
+constexpr long long kCountOne = 1ll << 56;
+constexpr long long kCountMark = 1ll << 47;
+
+template <int N>
+PSF_DEVINL void count_post(long long* words, long long (&w)[N], bool ok) {
+#pragma unroll
+  for (int q = 0; q + 1 < N; ++q) {  // limbs into [-2^47, 2^47)
+    const long long carry = (w[q] + (1ll << 47)) >> 48;
+    w[q] -= carry << 48;
+    w[q + 1] += carry;
+  }
+  if (!ok) w[N - 1] = kCountMark;
+#pragma unroll
+  for (int q = 0; q < N; ++q) red_add_s64(words + q, w[q] + kCountOne);
+}
+
+// One thread: waits (bounded) for G arrivals on each word; w the sums.
+template <int N>
+PSF_DEVINL bool count_wait(const long long* words, int G, long long (&w)[N], bool& ok, int* err) {
+  unsigned long long t0 = 0;
+  for (unsigned n = 0;; ++n) {
+    bool all = true;
+#pragma unroll
+    for (int q = 0; q < N; ++q) w[q] = ld_relaxed_s64(words + q);
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      const long long c = (long long)((unsigned long long)(w[q] + (1ll << 55)) >> 56);
+      all &= c == G;
+      w[q] -= (long long)((unsigned long long)c << 56);
+    }
+    if (all) break;
+    if ((n & 63u) == 63u) {
+      if (t0 == 0) t0 = globaltimer_ns();
+      if (*(volatile int*)err != 0) return false;
+      if (globaltimer_ns() - t0 > kWaitLimitNs) {
+        atomicOr(err, DEVERR_TIMEOUT);
+        return false;
+      }
+    }
+  }
+  ok = w[N - 1] < (1ll << 46) && w[N - 1] > -(1ll << 46);
+  return true;
+}
+
 }  // namespace psf

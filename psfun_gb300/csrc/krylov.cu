@@ -62,6 +62,11 @@ struct KState {
 constexpr int kVecThreads = 256;
 constexpr int kDenseThreads = 256;
 constexpr int kMgsThreads = 1024;
+// The words of the Lanczos reductions (fixsum.cuh) in KState::partials (2 x 4096
+// doubles): three buffers that the steps use in turn, each the two limbs of
+// alpha, CTA 0's answer to a stop request and the four limbs of the norm on a
+// 64-byte line.
+constexpr int kLzWordsAt = 4096, kLzBuf = 8, kLzWords = 3 * kLzBuf;
 
 // ---------------------------------------------------------------------------
 // kernels
@@ -88,6 +93,8 @@ __global__ void __launch_bounds__(kVecThreads) k_init(KState st, const double* _
   __shared__ double red[32];
   double* w1 = WAT(st, 1);
   double acc = 0.0;
+  // the sums of the Lanczos reductions start at zero
+  if (blockIdx.x == 0 && threadIdx.x < kLzWords) st.partials[kLzWordsAt + threadIdx.x] = 0.0;
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < st.n; r += (int64_t)gridDim.x * blockDim.x) {
     const double v = x[r];
     w1[r] = v;
@@ -114,11 +121,18 @@ __global__ void __launch_bounds__(kVecThreads) k_init(KState st, const double* _
 // Each CTA owns a contiguous range of row tiles (static schedule: the tile
 // after next is staged by TMA while the current one is computed).  Per step:
 //   phase 1  u = A W_i on the CTA's rows, partial W_i . u
-//   barrier  every CTA sums the partials in the same order -> alpha_i
+//   reduce   every CTA sums the partials in the same order -> alpha_i (no
+//            fence: phase 2 touches the CTA's own rows only)
 //   phase 2  W_{i+1} = 2^k (u - alpha W_i - c2 W_{i-1}), partial ||.||^2
-//   barrier  every CTA sums -> beta_{i+1}, s_{i+1}
-// Every CTA derives the scalars itself, so none is re-read from memory, and
-// CTA 0 records H, s and itx for the estimate / final kernels.
+//   reduce   every CTA sums -> beta_{i+1}, s_{i+1}; with fences, as the next
+//            SpMV reads W_{i+1} of other CTAs
+// (fixed-point sums that count their arrivals, fixsum.cuh).  Every CTA derives
+// the scalars itself, so none is re-read from memory, and CTA 0 records H, s
+// and itx for the estimate / final kernels.  The bounds of the sums come from
+// ||A||_2 <= 2^ea: |W.u| <= 2^ea ||W||^2, and ||w|| <= 5 2^ea ||W|| as c2 W_{i-1}
+// is the previous step's ||w|| long; ||W|| = 1 / s_i.  Measured:
+// 100 x 100, istop 1: 0.321 -> 0.298 ms; multi-shift on 96^3, 438 steps: 15.03 ->
+// 14.61; the steps of 512 x 512: 13.8 -> 12.6 us.
 // ---------------------------------------------------------------------------
 // Shifts of a multi-shift solve on one Lanczos basis (quadrature sums and
 // the adjoint): (xi_j I + sign T) is monitored by the LDL^T recurrences.
@@ -176,14 +190,13 @@ __device__ __noinline__ void est_monitor_cta(KState& st, const LzMonitor& mon, i
 
 // MODE LZ_PLAIN: the grid is the compute CTAs.  Otherwise the grid has
 // lz_monitors<MODE>() more blocks, the monitors.  The steps read a monitor's stop request through
-// CTA 0: its thread 0 copies stop_req into stop_dec before arriving at the
-// first grid barrier of a step, and every CTA reads stop_dec after that
-// barrier, so all of them leave at the same step.  Steps run past the one at
+// CTA 0: it reads stop_req at the start of a step and posts the answer (tagged
+// with the step) beside the sums, so all of them leave at the same step.  Steps run past the one at
 // which the monitor decides change nothing it uses (they write later basis
 // slots and T entries).
 template <int MODE>
 __global__ void __launch_bounds__(kSpmvThreads) k_lz_persist(KState st, CsrDev A, int i_begin, int i_end,
-                                                             int tiles_per_cta, LzMonitor mon) {
+                                                             int tiles_per_cta, int ea, LzMonitor mon) {
   extern __shared__ __align__(128) unsigned char lz_smem_raw[];
   LzSmem& sm = *reinterpret_cast<LzSmem*>(lz_smem_raw);
   constexpr bool kMon = MODE != LZ_PLAIN;
@@ -214,9 +227,9 @@ __global__ void __launch_bounds__(kSpmvThreads) k_lz_persist(KState st, CsrDev A
     if (!pipe_produce(A, t0, t0 + min(kLzStages, t1 - t0), sm, pc.issued, stream))
       atomicOr(&c->err, DEVERR_TIMEOUT);
   }
-  double sc = st.s[i_begin];       // s_i (thread 0 keeps it current; others read it after each barrier)
-  double wn_prev = 0.0;            // thread 0: ||W_i|| and k of the previous step
-  int k2_prev = 0;
+  double sc = st.s[i_begin];  // s_i (formed by the scalar thread; others read it after each reduction)
+  int k2 = 0;                 // floor(log2 s) of the previous step
+  long long* const words = reinterpret_cast<long long*>(st.partials + kLzWordsAt);
   double sprev = (i_begin >= 2) ? st.s[i_begin - 1] : 0.0;
   double beta_i = (i_begin >= 2) ? HAT(st, i_begin - 1, i_begin) : 0.0;
   double* __restrict__ u = st.u;
@@ -226,45 +239,77 @@ __global__ void __launch_bounds__(kSpmvThreads) k_lz_persist(KState st, CsrDev A
     const double* __restrict__ wi = WAT(st, i);
     // ---- phase 1
     double acc = 0.0;
-    // The per-step scalars are formed by thread 0 and broadcast through shared
-    // memory: a division or square root costs about ten dependent FP64
+    // The per-step scalars are formed by one thread and broadcast through
+    // shared memory: a division or square root costs about ten dependent FP64
     // instructions, which every warp would otherwise repeat on the critical
-    // path after each grid barrier.  What does not depend on this step's sums
+    // path after each reduction.  What does not depend on this step's sums
     // (c2, and s_i = 1 / (2^k ||W_i||) of the previous step) is formed at the
-    // start of the SpMV phase, where the other warps' work hides it.
-    if (threadIdx.x == 0) {
+    // start of the SpMV phase by a lane of the producer warp, which has tiles
+    // in flight then: the consumer warps do not wait for it.
+    if (threadIdx.x == kConsumerWarps * 32 + 1) {
+      if (kMon && bid == 0) *(volatile long long*)(words + (i % 3) * kLzBuf + 2) = 2ll * i + (*(volatile int*)&c->stop_req != 0);
       if (i > i_begin) {
-        sc = 1.0 / ldexp(wn_prev, k2_prev);
+        sc = 1.0 / ldexp(sm.scal[5], k2);
         if (bid == 0) st.s[i] = sc;
       }
       sm.scal[0] = sc;
       sm.scal[1] = (i >= 2) ? beta_i * sprev / sc : 0.0;
     }
+    __syncwarp();
     {
       EpiLzDot epi{u, wi, 0.0};
       pipe_spmv(A, wi, t0, t1, sm, epi, &c->err, pc, i + 1 < i_end, stream);
       acc = epi.acc;
     }
-    if (kMon && bid == 0 && threadIdx.x == 0) c->stop_dec = *(volatile int*)&c->stop_req;
-    block_sum_store_512(acc, sm.vals, sm.red, &st.partials[bid]);
-    if (!grid_sync_to(&c->bar_count, (unsigned)(2 * i - 1) * (unsigned)G, &c->err)) {
-      drain(i - i_begin + 1);
-      return;
-    }
+    long long* const acc_w = words + (i % 3) * kLzBuf;
     {
-      const double S = partials_sum_to0(st.partials, G, sm.red);
+      double S = 0.0, stop = 0.0;
+      block_sum_store_512(acc, sm.vals, sm.red, &S);
+      bool up = true;
       if (threadIdx.x == 0) {
+        sc = sm.scal[0];
+        const int E = ea - 2 * ilog2_normal(sc) + 4;
+        long long w[2];
+        bool ok;
+        {
+          int b[4];
+          ok = fix96_pieces(S, E, b);
+          w[0] = (long long)b[0] + ((long long)b[1] << 24);
+          w[1] = (long long)b[2] + ((long long)b[3] << 24);
+        }
+        count_post(acc_w, w, ok);
+        if (kMon) {  // CTA 0's answer has long been there when the sum completes
+          up = count_wait(acc_w, G, w, ok, &c->err);
+          long long d;
+          const unsigned long long t0 = globaltimer_ns();
+          while (up && ((d = *(volatile long long*)(acc_w + 2)) >> 1) != i) {
+            if (globaltimer_ns() - t0 > kWaitLimitNs) {
+              atomicOr(&c->err, DEVERR_TIMEOUT);
+              up = false;
+            }
+          }
+          stop = up && (d & 1) ? 1.0 : 0.0;
+        } else {
+          up = count_wait(acc_w, G, w, ok, &c->err);
+        }
+        S = ok ? fix96_value(w[1], w[0], E) : __longlong_as_double(0x7ff8000000000000ll);
         const double a = sc * sc * S;
         sm.scal[2] = a;
-        const int stop = kMon ? *(volatile int*)&c->stop_dec : 0;
-        sm.scal[4] = stop ? 1.0 : 0.0;
-        if (bid == 0 && !stop) {
+        sm.scal[4] = stop;
+        // the next step's words start at zero: every CTA has read what they
+        // held two steps ago, and adds to them after this CTA's next post
+        if (bid == 0)
+          for (int q = 0; q < kLzBuf; ++q) words[((i + 1) % 3) * kLzBuf + q] = 0;
+        if (bid == 0 && stop == 0.0) {
           HAT(st, i, i) = a;
           if (i >= 2) c->itx = i - 1;
         }
       }
+      if (__syncthreads_or(!up)) {
+        drain(i - i_begin + 1);
+        return;
+      }
     }
-    __syncthreads();
     if (kMon && sm.scal[4] != 0.0) {  // the monitor has decided: leave before the update
       drain(i - i_begin + 1);
       return;
@@ -273,7 +318,7 @@ __global__ void __launch_bounds__(kSpmvThreads) k_lz_persist(KState st, CsrDev A
     const double alpha = sm.scal[2];
     const double c2 = sm.scal[1];
     // ---- phase 2
-    const int k2 = ilog2_normal(sc);
+    k2 = ilog2_normal(sc);
     const double* __restrict__ wm = (i >= 2) ? WAT(st, i - 1) : wi;
     double* __restrict__ wo = WAT(st, i + 1);
     // four rows per thread in flight: the loads of a group are issued before
@@ -301,19 +346,23 @@ __global__ void __launch_bounds__(kSpmvThreads) k_lz_persist(KState st, CsrDev A
       acc2 = fma(w, w, acc2);
       wo[r] = scale_pow2(w, k2);
     }
-    block_sum_store_512(acc2, sm.vals, sm.red, &st.partials[G + bid]);
-    if (!grid_sync_to(&c->bar_count, (unsigned)(2 * i) * (unsigned)G, &c->err)) {
-      drain(i - i_begin + 1);
-      return;
-    }
     {
-      const double S = partials_sum_to0(st.partials + G, G, sm.red);
+      double S = 0.0;
+      block_sum_store_512(acc2, sm.vals, sm.red, &S);
+      bool up = true;
       if (threadIdx.x == 0) {
+        const int E = 2 * (ea - k2 + 3) + 4;
+        long long w[4];
+        bool ok = fix192_limbs(S, E, w);
+        __threadfence();  // the block's rows of W_{i+1}, ordered before by block_sum_store_512's barriers
+        count_post(acc_w + 4, w, ok);
+        up = count_wait(acc_w + 4, G, w, ok, &c->err);
+        __threadfence();
+        S = ok ? fix192_value(w[3], w[2], w[1], w[0], E) : __longlong_as_double(0x7ff8000000000000ll);
         const double wn = sqrt(S);
         const double bt = sc * wn;
         sm.scal[3] = bt;
-        wn_prev = wn;
-        k2_prev = k2;
+        sm.scal[5] = wn;
         if (bid == 0) {
           HAT(st, i, i + 1) = bt;
           HAT(st, i + 1, i) = bt;
@@ -328,12 +377,15 @@ __global__ void __launch_bounds__(kSpmvThreads) k_lz_persist(KState st, CsrDev A
           }
         }
       }
+      if (__syncthreads_or(!up)) {
+        drain(i - i_begin + 1);
+        return;
+      }
     }
-    __syncthreads();
     const double beta = sm.scal[3];
     if (i + 1 <= st.nl && fabs(beta) < 1e-16) {  // checked at the top of iteration i+1
       if (bid == 0 && threadIdx.x == 0) {
-        st.s[i + 1] = 1.0 / ldexp(wn_prev, k2_prev);
+        st.s[i + 1] = 1.0 / ldexp(sm.scal[5], k2);
         c->bd_step = i;
         c->breakdown = 1;
         c->itx = i;
@@ -345,7 +397,7 @@ __global__ void __launch_bounds__(kSpmvThreads) k_lz_persist(KState st, CsrDev A
     beta_i = beta;
   }
   // s of the last vector, formed ahead of the next step in the loop above
-  if (bid == 0 && threadIdx.x == 0) st.s[i_end] = 1.0 / ldexp(wn_prev, k2_prev);
+  if (bid == 0 && threadIdx.x == 0) st.s[i_end] = 1.0 / ldexp(sm.scal[5], k2);
 }
 
 // Arnoldi: w = scaling * A v_{i-1} into slot i through the warp-specialised
@@ -1315,30 +1367,34 @@ static int persist_grid() {
 // Steps [i_begin, i_end) in one cooperative launch; with a monitor the grid
 // holds the compute CTAs and the monitor block.
 template <int MODE>
-static int launch_lz_persist_mode(KState& st, const CsrDev& A, int i_begin, int i_end, const LzMonitor& mon,
-                                  cudaStream_t s) {
+static int launch_lz_persist_mode(KState& st, const CsrDev& A, double norm_inf, int i_begin, int i_end,
+                                  const LzMonitor& mon, cudaStream_t s) {
   const int extra = lz_monitors<MODE>();
   int G = persist_grid<MODE>() - extra;
   if (G < 1) {
     set_last_error("persistent Lanczos: no room for the monitor blocks");
     return PSFUN_ERR_CUDA;
   }
+  G = std::min(G, kCountMaxBlocks);
   int tpc = (A.ntiles + G - 1) / G;
   if (tpc < 1) tpc = 1;
   G = (A.ntiles + tpc - 1) / tpc;
   if (G < 1) G = 1;
   LzMonitor m = mon;
-  void* args[] = {(void*)&st, (void*)&A, (void*)&i_begin, (void*)&i_end, (void*)&tpc, (void*)&m};
+  // ||A||_2 <= sqrt(n) ||A||_inf < 2^ea (a symmetric A needs no sqrt(n), but the method does not ask for one)
+  const double bound = norm_inf * std::sqrt((double)std::max<int64_t>(st.n, 1));
+  int ea = bound > 0.0 ? (std::isfinite(bound) ? std::ilogb(bound) + 1 : 1000) : 0;
+  void* args[] = {(void*)&st, (void*)&A, (void*)&i_begin, (void*)&i_end, (void*)&tpc, (void*)&ea, (void*)&m};
   PSF_CUDA(cudaLaunchCooperativeKernel((void*)k_lz_persist<MODE>, dim3(G + extra), dim3(kSpmvThreads), args,
                                        kLzSmemBytes, s));
   count_launch();
   return PSFUN_SUCCESS;
 }
 
-static int launch_lz_persist(KState& st, const CsrDev& A, int i_begin, int i_end, cudaStream_t s) {
+static int launch_lz_persist(KState& st, const CsrDev& A, double norm_inf, int i_begin, int i_end, cudaStream_t s) {
   LzMonitor none;
   memset(&none, 0, sizeof none);
-  return launch_lz_persist_mode<LZ_PLAIN>(st, A, i_begin, i_end, none, s);
+  return launch_lz_persist_mode<LZ_PLAIN>(st, A, norm_inf, i_begin, i_end, none, s);
 }
 
 static int grid_for(int64_t items, int threads, int per_sm) {
@@ -1502,7 +1558,7 @@ int krylov_apply_device(psfun_krylov* meth, psfun_serial* fun, psfun_csr* a, dou
     PSF_CUDA(cudaGetLastError());
     if (!arnoldi && lz_step1) {
       prof_begin(PROF_LZ_SPMV, s);
-      PSF_TRY(launch_lz_persist(st, A, 1, 2, s));
+      PSF_TRY(launch_lz_persist(st, A, a->norm_inf, 1, 2, s));
       prof_end(PROF_LZ_SPMV, s);
     }
     return PSFUN_SUCCESS;
@@ -1544,7 +1600,7 @@ int krylov_apply_device(psfun_krylov* meth, psfun_serial* fun, psfun_csr* a, dou
       count_launch((sai || fuse_spmv) ? 1 : 2);
     } else {
       prof_begin(PROF_LZ_SPMV, s);
-      PSF_TRY(launch_lz_persist(st, A, i, i + 1, s));
+      PSF_TRY(launch_lz_persist(st, A, a->norm_inf, i, i + 1, s));
       prof_end(PROF_LZ_SPMV, s);
     }
     PSF_CUDA(cudaGetLastError());
@@ -1621,7 +1677,7 @@ int krylov_apply_device(psfun_krylov* meth, psfun_serial* fun, psfun_csr* a, dou
     mon.scr = lz_scr;
     mon.scr_stride = lz_scr_stride;
     mon.count = kEstMonitors;
-    PSF_TRY(launch_lz_persist_mode<LZ_MON_ESTIMATE>(st, A, 1, nl + 1, mon, s));
+    PSF_TRY(launch_lz_persist_mode<LZ_MON_ESTIMATE>(st, A, a->norm_inf, 1, nl + 1, mon, s));
     k_par_select<<<1, kDenseThreads, 0, s>>>(st, lz_yk_all, nl + 1, -1);
     count_launch();
     PSF_CUDA(cudaGetLastError());
@@ -1682,7 +1738,7 @@ int krylov_apply_device(psfun_krylov* meth, psfun_serial* fun, psfun_csr* a, dou
       PSF_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
       int rc = enqueue_prologue(false);
       if (!arnoldi) {
-        if (rc == PSFUN_SUCCESS) rc = lz_mon ? launch_lz_estimating() : launch_lz_persist(st, A, 1, nl + 1, s);
+        if (rc == PSFUN_SUCCESS) rc = lz_mon ? launch_lz_estimating() : launch_lz_persist(st, A, a->norm_inf, 1, nl + 1, s);
       } else if (cwy.G > 0) {
         if (rc == PSFUN_SUCCESS) rc = launch_cwy();
       } else {
@@ -1706,7 +1762,7 @@ int krylov_apply_device(psfun_krylov* meth, psfun_serial* fun, psfun_csr* a, dou
     // the graph, timed under the Lanczos slot
     PSF_TRY(enqueue_prologue(false));
     prof_begin(PROF_LZ_SPMV, s);
-    PSF_TRY(lz_mon ? launch_lz_estimating() : launch_lz_persist(st, A, 1, nl + 1, s));
+    PSF_TRY(lz_mon ? launch_lz_estimating() : launch_lz_persist(st, A, a->norm_inf, 1, nl + 1, s));
     prof_end(PROF_LZ_SPMV, s);
     PSF_TRY(enqueue_epilogue(0));
   } else {
@@ -2144,7 +2200,7 @@ static int shifted_lanczos(psfun_krylov* ws, DevBuf& msbuf, psfun_csr* a, const 
   LzMonitor mon;
   memset(&mon, 0, sizeof mon);
   mon.mp = mp;
-  PSF_TRY(launch_lz_persist_mode<LZ_MON_SHIFTS>(st, A, 1, nl + 1, mon, s));
+  PSF_TRY(launch_lz_persist_mode<LZ_MON_SHIFTS>(st, A, a->norm_inf, 1, nl + 1, mon, s));
   PSF_CUDA(cudaGetLastError());
   KCtrl hc;
   int hmon = 0;
