@@ -225,9 +225,10 @@ __global__ void k_diag_inv(int64_t n, const double* d, double* out) {
 //   x += alpha p, r -= alpha q, z = D r, partial r.z and the norms of the
 //   stopping rule                                      -> barrier -> stop, beta
 // Thread 0 of every block forms the same scalars from the per-block partials
-// in the same order; block 0 records them in the control block.  The maxima of the stopping rule are taken as integers
-// of the values' bits (two FP64 maxima per row would be a third of the update's
-// time on the FP64 pipe).  @@CG@@  The kernel
+// in the same order; block 0 records them in the control block.  The maxima of
+// the stopping rule are taken as integers of the values' bits (two FP64 maxima
+// per row would be a third of the update's FP64 instructions; 128^3, DIAG: 5.23
+// -> 5.02 ms).  The kernel
 // returns when the stopping rule holds, itx reaches itmax, or a breakdown
 // (sigma = 0 or rho_old = 0) asks the host to restart.
 // ---------------------------------------------------------------------------

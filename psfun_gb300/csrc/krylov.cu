@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kVecThreads) k_init(KState st, const double* _
 // ||A||_2 <= 2^ea: |W.u| <= 2^ea ||W||^2, and ||w|| <= 5 2^ea ||W|| as c2 W_{i-1}
 // is the previous step's ||w|| long; ||W|| = 1 / s_i.  Measured:
 // 100 x 100, istop 1: 0.321 -> 0.298 ms; multi-shift on 96^3, 438 steps: 15.03 ->
-// 14.61; the steps of 512 x 512: 13.8 -> 12.6 us.
+// 14.61.
 // ---------------------------------------------------------------------------
 // Shifts of a multi-shift solve on one Lanczos basis (quadrature sums and
 // the adjoint): (xi_j I + sign T) is monitored by the LDL^T recurrences.
@@ -201,18 +201,19 @@ __global__ void __launch_bounds__(kSpmvThreads) k_lz_persist(KState st, CsrDev A
   LzSmem& sm = *reinterpret_cast<LzSmem*>(lz_smem_raw);
   constexpr bool kMon = MODE != LZ_PLAIN;
   KCtrl* c = st.ctrl;
-  if (c->done) return;
+  const int G = gridDim.x - lz_monitors<MODE>(), bid = blockIdx.x;
+  // (block-wide decisions on words that a step already running may change)
+  if (__syncthreads_or(c->done)) return;
+  if (kMon && bid >= G) {
+    if (MODE == LZ_MON_SHIFTS) ms_monitor_cta(st, mon.mp, i_begin, i_end);
+    else est_monitor_cta(st, mon, i_begin, i_end, bid - G);
+    return;
+  }
   if (c->breakdown) {  // found by the previous launch: exit at the top of iteration i_begin
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       c->done = 1;
       if (st.host_flag) st.host_flag[0] = 1;
     }
-    return;
-  }
-  const int G = gridDim.x - lz_monitors<MODE>(), bid = blockIdx.x;
-  if (kMon && bid >= G) {
-    if (MODE == LZ_MON_SHIFTS) ms_monitor_cta(st, mon.mp, i_begin, i_end);
-    else est_monitor_cta(st, mon, i_begin, i_end, bid - G);
     return;
   }
   lz_smem_init(sm);
@@ -821,8 +822,9 @@ __device__ void estimate_body(KState& st, const FunParams& fp, int i, double eps
   KCtrl* c = st.ctrl;
   if (st.errn_all) {
     // concurrent estimates: skip only when an estimate of an earlier
-    // iteration has converged (c->done can be set by a later step meanwhile)
-    if (*(volatile int*)&c->conv_first < i || c->beta0 == 0.0) return;
+    // iteration has converged (c->done can be set by a later step meanwhile).
+    // The word changes while the block reads it: the block decides as one.
+    if (__syncthreads_or(*(volatile int*)&c->conv_first < i || c->beta0 == 0.0)) return;
   } else if (c->done) {
     return;
   }
@@ -1037,7 +1039,8 @@ __device__ __noinline__ void est_monitor_cta(KState& st, const LzMonitor& mon, i
     estimate_body(ste, mon.fp, i, mon.eps, mon.tridiag, dsm, false);
     __syncthreads();
     if (threadIdx.x == 0) atomicMax(&c->est_last, i);
-    if (*(volatile int*)&c->info != 0 || *(volatile int*)&c->conv_first <= i) return;
+    // as one: warps that left alone would be missing from the next estimate's barriers
+    if (__syncthreads_or(*(volatile int*)&c->info != 0 || *(volatile int*)&c->conv_first <= i)) return;
   }
 }
 
