@@ -195,13 +195,12 @@ __device__ __noinline__ void est_monitor_cta(KState& st, const LzMonitor& mon, i
 // which the monitor decides change nothing it uses (they write later basis
 // slots and T entries).
 template <int MODE>
-__global__ void __launch_bounds__(kSpmvThreads) k_lz_persist(KState st, CsrDev A, int i_begin, int i_end,
-                                                             int tiles_per_cta, int ea, LzMonitor mon) {
+PSF_DEVINL void lz_persist_body(KState& st, const CsrDev& A, int i_begin, int i_end, int tiles_per_cta, int ea,
+                                const LzMonitor& mon, int bid, int G) {
   extern __shared__ __align__(128) unsigned char lz_smem_raw[];
   LzSmem& sm = *reinterpret_cast<LzSmem*>(lz_smem_raw);
   constexpr bool kMon = MODE != LZ_PLAIN;
   KCtrl* c = st.ctrl;
-  const int G = gridDim.x - lz_monitors<MODE>(), bid = blockIdx.x;
   // (block-wide decisions on words that a step already running may change)
   if (__syncthreads_or(c->done)) return;
   if (kMon && bid >= G) {
@@ -210,7 +209,7 @@ __global__ void __launch_bounds__(kSpmvThreads) k_lz_persist(KState st, CsrDev A
     return;
   }
   if (c->breakdown) {  // found by the previous launch: exit at the top of iteration i_begin
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (bid == 0 && threadIdx.x == 0) {
       c->done = 1;
       if (st.host_flag) st.host_flag[0] = 1;
     }
@@ -399,6 +398,25 @@ __global__ void __launch_bounds__(kSpmvThreads) k_lz_persist(KState st, CsrDev A
   }
   // s of the last vector, formed ahead of the next step in the loop above
   if (bid == 0 && threadIdx.x == 0) st.s[i_end] = 1.0 / ldexp(sm.scal[5], k2);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kSpmvThreads) k_lz_persist(KState st, CsrDev A, int i_begin, int i_end,
+                                                             int tiles_per_cta, int ea, LzMonitor mon) {
+  lz_persist_body<MODE>(st, A, i_begin, i_end, tiles_per_cta, ea, mon, blockIdx.x, gridDim.x - lz_monitors<MODE>());
+}
+
+// Two multi-shift solves with one matrix (the adjoint's bases of x and g), each
+// on every second block with a monitor of its own.  Below ~600 thousand rows
+// more than half of a step is latency (reductions over the grid, the start of
+// the SpMV), which the two solves pay at the same time.  Grid graph 512 x 512:
+// forward and backward 1.185 -> 0.965 ms.
+__global__ void __launch_bounds__(kSpmvThreads) k_lz_pair(KState sx, KState sg, CsrDev A, int i_end, int tiles_per_cta,
+                                                          int ea, LzMonitor mx, LzMonitor mg) {
+  const bool second = (blockIdx.x & 1) != 0;
+  KState st = second ? sg : sx;
+  const LzMonitor mon = second ? mg : mx;
+  lz_persist_body<LZ_MON_SHIFTS>(st, A, 1, i_end, tiles_per_cta, ea, mon, blockIdx.x >> 1, (gridDim.x >> 1) - 1);
 }
 
 // Arnoldi: w = scaling * A v_{i-1} into slot i through the warp-specialised
@@ -1367,6 +1385,13 @@ static int persist_grid() {
   return g;
 }
 
+// ||A||_2 <= sqrt(n) ||A||_inf < 2^ea (a symmetric A needs no sqrt(n), but the
+// method does not ask for one).
+static int lz_norm_exponent(double norm_inf, int64_t n) {
+  const double bound = norm_inf * std::sqrt((double)std::max<int64_t>(n, 1));
+  return bound > 0.0 ? (std::isfinite(bound) ? std::ilogb(bound) + 1 : 1000) : 0;
+}
+
 // Steps [i_begin, i_end) in one cooperative launch; with a monitor the grid
 // holds the compute CTAs and the monitor block.
 template <int MODE>
@@ -1384,9 +1409,7 @@ static int launch_lz_persist_mode(KState& st, const CsrDev& A, double norm_inf, 
   G = (A.ntiles + tpc - 1) / tpc;
   if (G < 1) G = 1;
   LzMonitor m = mon;
-  // ||A||_2 <= sqrt(n) ||A||_inf < 2^ea (a symmetric A needs no sqrt(n), but the method does not ask for one)
-  const double bound = norm_inf * std::sqrt((double)std::max<int64_t>(st.n, 1));
-  int ea = bound > 0.0 ? (std::isfinite(bound) ? std::ilogb(bound) + 1 : 1000) : 0;
+  int ea = lz_norm_exponent(norm_inf, st.n);
   void* args[] = {(void*)&st, (void*)&A, (void*)&i_begin, (void*)&i_end, (void*)&tpc, (void*)&ea, (void*)&m};
   PSF_CUDA(cudaLaunchCooperativeKernel((void*)k_lz_persist<MODE>, dim3(G + extra), dim3(kSpmvThreads), args,
                                        kLzSmemBytes, s));
@@ -2134,9 +2157,10 @@ struct ShiftedRun {
   double err;
 };
 
-static int shifted_lanczos(psfun_krylov* ws, DevBuf& msbuf, psfun_csr* a, const double* b, int N,
-                           const double* xi_host, const double* c_host, double sign, double eps, int itmax,
-                           ShiftedRun* out) {
+// Workspace, shifts and the first vector of a multi-shift solve, up to the
+// launch of its steps.
+static int shifted_begin(psfun_krylov* ws, DevBuf& msbuf, psfun_csr* a, const double* b, int N, const double* xi_host,
+                         const double* c_host, double sign, double eps, int itmax, ShiftedRun* out) {
   const int64_t n = a->n;
   const int nl = itmax;
   PSF_TRY(ensure_workspace(ws, n, nl, 1));
@@ -2191,30 +2215,72 @@ static int shifted_lanczos(psfun_krylov* ws, DevBuf& msbuf, psfun_csr* a, const 
   hflag[0] = 0;
   hflag[1] = 0;
   st.host_flag = dflag;
-  const CsrDev A = a->dev();
   spmv_kernel_attrs();
   const int gv = vec_grid(n);
   k_init<<<gv, kVecThreads, 0, s>>>(st, b);
   count_launch();
-  // Every Lanczos step in one persistent cooperative launch; its monitor
-  // block advances the shifted recurrences as the steps are published and
-  // stops the steps at the first step at which every shift has converged.
   PSF_CUDA(cudaMemsetAsync(mp.mon, 0, sizeof(int), s));
-  LzMonitor mon;
-  memset(&mon, 0, sizeof mon);
-  mon.mp = mp;
-  PSF_TRY(launch_lz_persist_mode<LZ_MON_SHIFTS>(st, A, a->norm_inf, 1, nl + 1, mon, s));
-  PSF_CUDA(cudaGetLastError());
+  return PSFUN_SUCCESS;
+}
+
+// Waits for the steps and takes their outcome.
+static int shifted_end(ShiftedRun* out) {
+  cudaStream_t s = stream();
   KCtrl hc;
   int hmon = 0;
-  PSF_CUDA(cudaMemcpyAsync(&hc, st.ctrl, sizeof hc, cudaMemcpyDeviceToHost, s));
-  PSF_CUDA(cudaMemcpyAsync(&hmon, mp.mon, sizeof(int), cudaMemcpyDeviceToHost, s));
+  PSF_CUDA(cudaMemcpyAsync(&hc, out->st.ctrl, sizeof hc, cudaMemcpyDeviceToHost, s));
+  PSF_CUDA(cudaMemcpyAsync(&hmon, out->mp.mon, sizeof(int), cudaMemcpyDeviceToHost, s));
   PSF_CUDA(cudaStreamSynchronize(s));
   if (hc.err & DEVERR_TIMEOUT) return PSFUN_ERR_DEVICE_TIMEOUT;
   if (hc.info != 0) return hc.info;
   out->m = hmon;
   out->err = hc.errnum;
   return PSFUN_SUCCESS;
+}
+
+static int shifted_lanczos(psfun_krylov* ws, DevBuf& msbuf, psfun_csr* a, const double* b, int N,
+                           const double* xi_host, const double* c_host, double sign, double eps, int itmax,
+                           ShiftedRun* out) {
+  PSF_TRY(shifted_begin(ws, msbuf, a, b, N, xi_host, c_host, sign, eps, itmax, out));
+  // Every Lanczos step in one persistent cooperative launch; its monitor
+  // block advances the shifted recurrences as the steps are published and
+  // stops the steps at the first step at which every shift has converged.
+  LzMonitor mon;
+  memset(&mon, 0, sizeof mon);
+  mon.mp = out->mp;
+  PSF_TRY(launch_lz_persist_mode<LZ_MON_SHIFTS>(out->st, a->dev(), a->norm_inf, 1, itmax + 1, mon, stream()));
+  PSF_CUDA(cudaGetLastError());
+  return shifted_end(out);
+}
+
+// Whether two solves run as one launch (k_lz_pair): up to eight tiles per
+// block of a solve alone; above, the FP64 pipe bounds a step and the halves of
+// the grid only make its shares less even.
+static bool lz_pair_pays(const psfun_csr* a) { return a->ntiles <= 8 * sm_count() && sm_count() >= 8; }
+
+static int shifted_pair(psfun_krylov* wx, psfun_krylov* wg, DevBuf& msx, DevBuf& msg, psfun_csr* a, const double* x,
+                        const double* g, int N, const double* xi_host, double sign, double eps, int itmax,
+                        ShiftedRun* rx, ShiftedRun* rg) {
+  PSF_TRY(shifted_begin(wx, msx, a, x, N, xi_host, nullptr, sign, eps, itmax, rx));
+  PSF_TRY(shifted_begin(wg, msg, a, g, N, xi_host, nullptr, sign, eps, itmax, rg));
+  static const int blocks = persist_grid_for(k_lz_pair);
+  const int half = std::min(blocks / 2 - 1, kCountMaxBlocks);
+  int tpc = std::max(1, (a->ntiles + half - 1) / half);
+  const int G = std::max(1, (a->ntiles + tpc - 1) / tpc);
+  int ea = lz_norm_exponent(a->norm_inf, a->n), i_end = itmax + 1;
+  CsrDev A = a->dev();
+  LzMonitor mx, mg;
+  memset(&mx, 0, sizeof mx);
+  memset(&mg, 0, sizeof mg);
+  mx.mp = rx->mp;
+  mg.mp = rg->mp;
+  void* args[] = {(void*)&rx->st, (void*)&rg->st, (void*)&A,  (void*)&i_end,
+                  (void*)&tpc,    (void*)&ea,     (void*)&mx, (void*)&mg};
+  PSF_CUDA(cudaLaunchCooperativeKernel((void*)k_lz_pair, dim3(2 * (G + 1)), dim3(kSpmvThreads), args, kLzSmemBytes,
+                                       stream()));
+  count_launch();
+  PSF_TRY(shifted_end(rx));
+  return shifted_end(rg);
 }
 
 int quad_apply_device(psfun_csr* a, int N, const double* xi, const double* cw, double eta, double sign,
@@ -2283,8 +2349,17 @@ struct AdjShifts {
 
 // sol_k = (z_k I - t T(1:m))^{-1} beta0 e1 (banded GEPP, one thread per
 // shift); coef[p] = Re(sum_k c_k sol_k[p]) * s[p+1].
-__global__ void k_adj_solve(KState st, AdjShifts sh, int m, double* sol, double* band, double* coef,
-                            double* s_save) {
+struct AdjSide {
+  KState st;
+  int m;
+  double *sol, *band, *coef, *s_save;
+};
+
+__global__ void k_adj_solve(AdjSide s0, AdjSide s1, AdjShifts sh) {
+  const AdjSide& side = blockIdx.x == 0 ? s0 : s1;  // a block per basis
+  const KState st = side.st;
+  const int m = side.m;
+  double *sol = side.sol, *band = side.band, *coef = side.coef, *s_save = side.s_save;
   __shared__ int bad;
   if (threadIdx.x == 0) bad = 0;
   __syncthreads();
@@ -2692,12 +2767,12 @@ int expm_adjoint_device(psfun_csr* a, double t, const double* x, const double* g
   if (!wsx) wsx = new psfun_krylov();
   if (!wsg) wsg = new psfun_krylov();
   psfun_krylov* wg = recompute ? wsx : wsg;
-  static DevBuf msb, adj, pbuf, tmpv;
+  static DevBuf msb, msb2, adj, pbuf, tmpv;
   cudaStream_t s = stream();
   const int64_t n = a->n;
   const int64_t ld = (n + 31) & ~(int64_t)31;
   // small buffers: shifts, solutions, bands, coefficients, saved scales, R
-  const size_t nsmall = 4 * (size_t)Nq + 2 * (2 * (size_t)Nq * itmax) + 8 * (size_t)Nq * itmax + 4 * (size_t)itmax +
+  const size_t nsmall = 4 * (size_t)Nq + 2 * (2 * (size_t)Nq * itmax) + 2 * (8 * (size_t)Nq * itmax) + 4 * (size_t)itmax +
                         2 * (size_t)(itmax + 2) + (size_t)itmax * itmax + 4096 + 64;
   PSF_TRY(adj.ensure(sizeof(double) * nsmall));
   double* ab = adj.as<double>();
@@ -2706,7 +2781,8 @@ int expm_adjoint_device(psfun_csr* a, double t, const double* x, const double* g
   double* solx = dc + 2 * Nq;
   double* solg = solx + 2 * (size_t)Nq * itmax;
   double* band = solg + 2 * (size_t)Nq * itmax;
-  double* coefy = band + 8 * (size_t)Nq * itmax;
+  double* band2 = band + 8 * (size_t)Nq * itmax;
+  double* coefy = band2 + 8 * (size_t)Nq * itmax;
   double* coefg = coefy + itmax;
   double* sx = coefg + itmax;
   double* sg = sx + (itmax + 2);
@@ -2721,12 +2797,16 @@ int expm_adjoint_device(psfun_csr* a, double t, const double* x, const double* g
   double* ytmp = y ? y : tmpv.as<double>();
   double* Ay = tmpv.as<double>() + ld;
 
-  // forward basis (x): y = exp(tA) x
-  ShiftedRun rx;
-  PSF_TRY(shifted_lanczos(wsx, msb, a, x, Nq, xi_h.data(), nullptr, sign, eps, itmax, &rx));
+  // forward basis (x): y = exp(tA) x; with room for both bases, the adjoint's beside it
+  ShiftedRun rx, rg;
+  const bool pair = !recompute && (grad_x || grad_t || grad_vals) && lz_pair_pays(a);
+  if (pair) PSF_TRY(shifted_pair(wsx, wg, msb, msb2, a, x, g, Nq, xi_h.data(), sign, eps, itmax, &rx, &rg));
+  else PSF_TRY(shifted_lanczos(wsx, msb, a, x, Nq, xi_h.data(), nullptr, sign, eps, itmax, &rx));
   const int mx = rx.m;
   if (mx < 1) return PSFUN_ERR_FROM_SUBROUTINE_NON;
-  k_adj_solve<<<1, 32, 0, s>>>(rx.st, sh, mx, solx, band, coefy, sx);
+  const AdjSide ax{rx.st, mx, solx, band, coefy, sx};
+  if (pair && rg.m >= 1) k_adj_solve<<<2, 32, 0, s>>>(ax, AdjSide{rg.st, rg.m, solg, band2, coefg, sg}, sh);
+  else k_adj_solve<<<1, 32, 0, s>>>(ax, ax, sh);
   k_lincomb<<<grid_for(n, kVecThreads, 4), kVecThreads, 0, s>>>(rx.st.V, rx.st.ldv, n, coefy, mx, ytmp);
   count_launch(2);
   if (!grad_x && !grad_t && !grad_vals) {  // forward only
@@ -2739,12 +2819,16 @@ int expm_adjoint_device(psfun_csr* a, double t, const double* x, const double* g
     return PSFUN_SUCCESS;
   }
   // adjoint basis (g): dL/dx = exp(tA) g
-  ShiftedRun rg;
-  PSF_TRY(shifted_lanczos(wg, msb, a, g, Nq, xi_h.data(), nullptr, sign, eps, itmax, &rg));
+  if (!pair) {
+    PSF_TRY(shifted_lanczos(wg, msb, a, g, Nq, xi_h.data(), nullptr, sign, eps, itmax, &rg));
+    if (rg.m >= 1) {
+      const AdjSide ag{rg.st, rg.m, solg, band, coefg, sg};
+      k_adj_solve<<<1, 32, 0, s>>>(ag, ag, sh);
+      count_launch();
+    }
+  }
   const int mg = rg.m;
   if (mg < 1) return PSFUN_ERR_FROM_SUBROUTINE_NON;
-  k_adj_solve<<<1, 32, 0, s>>>(rg.st, sh, mg, solg, band, coefg, sg);
-  count_launch();
   if (grad_x) {
     k_lincomb<<<grid_for(n, kVecThreads, 4), kVecThreads, 0, s>>>(rg.st.V, rg.st.ldv, n, coefg, mg, grad_x);
     count_launch();
