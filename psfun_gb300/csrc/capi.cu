@@ -259,6 +259,32 @@ static void host_parallel_for(int64_t n, F f) {
   for (auto& x : th) x.join();
 }
 
+// The rows of each tile by descending length, equal lengths in row order: a
+// bitonic sort of (length, row) keys, one block per tile.
+__global__ void __launch_bounds__(256) k_tile_order(const int32_t* __restrict__ irp, const int2* __restrict__ desc,
+                                                    uint16_t* __restrict__ order) {
+  __shared__ unsigned key[512];
+  static_assert(kTileRows <= 512, "a tile's rows fit the sort");
+  const int r0 = desc[blockIdx.x].x, nr = desc[blockIdx.x + 1].x - r0;
+  for (int l = threadIdx.x; l < 512; l += blockDim.x) {
+    // 13 bits of length (a longer row is alone in its tile), 9 of row
+    const unsigned len = l < nr ? (unsigned)min(irp[r0 + l + 1] - irp[r0 + l], 8190) : 0u;
+    key[l] = l < nr ? (8191u - len) << 9 | (unsigned)l : 0xffffffffu;
+  }
+  for (int k = 2; k <= 512; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      __syncthreads();
+      const int a = 2 * threadIdx.x - (threadIdx.x & (j - 1)), b = a + j;
+      const unsigned x = key[a], y = key[b];
+      if ((x > y) == ((a & k) == 0)) {
+        key[a] = y;
+        key[b] = x;
+      }
+    }
+  __syncthreads();
+  for (int l = threadIdx.x; l < nr; l += blockDim.x) order[r0 + l] = (uint16_t)(key[l] & 511u);
+}
+
 extern "C" {
 
 int psfun_gpu_csr_create(int64_t n, int64_t nnz, const int32_t* irp, const int32_t* ja, const double* val,
@@ -341,12 +367,25 @@ int psfun_gpu_csr_create(int64_t n, int64_t nnz, const int32_t* irp, const int32
   std::mutex mx;
   double ninf = 0.0;
   int32_t max_row = 0;
+  // FP64 instructions that the plain schedule spends on 32 rows, near enough
+  // (warp_row_split with the threshold 32, groups counted from row 0)
+  int64_t cost = 0;
   host_parallel_for(n, [&](int64_t b, int64_t e) {
     double ninf_p = 0.0;
     int32_t max_row_p = 0;
+    int64_t cost_p = 0;
+    int lmax = 0, smax = 0, split = 0;
     for (int64_t i = b; i < e; ++i) {
       double s = 0.0;
-      max_row_p = std::max<int32_t>(max_row_p, hirp[i + 1] - hirp[i]);
+      const int len = hirp[i + 1] - hirp[i];
+      max_row_p = std::max<int32_t>(max_row_p, len);
+      lmax = std::max(lmax, len);
+      if (len > 32) split += (len + 31) / 32 + 5;
+      else smax = std::max(smax, len);
+      if ((i & 31) == 31 || i + 1 == e) {
+        cost_p += std::min(lmax, smax + split);
+        lmax = smax = split = 0;
+      }
       for (int32_t k = hirp[i]; k < hirp[i + 1]; ++k) {
         s += fabs(val[k]);
         if (hja[k] == i) a->h_diag[i] += val[k];
@@ -354,11 +393,17 @@ int psfun_gpu_csr_create(int64_t n, int64_t nnz, const int32_t* irp, const int32
       if (s > ninf_p) ninf_p = s;
     }
     std::lock_guard<std::mutex> lock(mx);
+    cost += cost_p;
     ninf = std::max(ninf, ninf_p);
     max_row = std::max(max_row, max_row_p);
   });
   a->norm_inf = ninf;
   a->max_row = max_row;
+  // An order by length pays where the plain schedule spends over 1.25 times the
+  // FP64 instructions of the entries: grid stencils (1.0 to 1.02) and most
+  // neighbour graphs lie below and keep their coalesced rows.  Below 2^15
+  // entries a product is all latency.
+  const bool ordered = (double)cost * 32.0 > 1.25 * (double)nnz && nnz >= ((int64_t)1 << 15);
   cudaStream_t s = stream();
   auto fail = [&](cudaError_t e) {
     (void)cudaGetLastError();
@@ -391,6 +436,13 @@ int psfun_gpu_csr_create(int64_t n, int64_t nnz, const int32_t* irp, const int32
   if ((e = cudaMemcpyAsync(a->tile_row, tiles.data(), sizeof(int32_t) * tiles.size(), cudaMemcpyHostToDevice, s)) !=
       cudaSuccess)
     return fail(e);
+  if (ordered) {
+    if ((e = cudaMalloc(&a->order, sizeof(uint16_t) * (n + 16))) != cudaSuccess) return fail(e);
+    if ((e = cudaMemsetAsync(a->order, 0, sizeof(uint16_t) * (n + 16), s)) != cudaSuccess) return fail(e);
+    k_tile_order<<<a->ntiles, 256, 0, s>>>(a->irp, a->tile_desc, a->order);
+    count_launch();
+    if ((e = cudaGetLastError()) != cudaSuccess) return fail(e);
+  }
   if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail(e);
   *out = a;
   return PSFUN_SUCCESS;
@@ -401,6 +453,7 @@ int psfun_gpu_csr_destroy(psfun_csr* a) {
   if (a->T) psfun_gpu_csr_destroy(a->T);
   if (a->bj_val) cudaFree(a->bj_val);
   if (a->bj_tri) cudaFree(a->bj_tri);
+  if (a->order) cudaFree(a->order);
   if (a->bj_col) cudaFree(a->bj_col);
   if (a->bj_rowoff) cudaFree(a->bj_rowoff);
   if (a->bj_cnt) cudaFree(a->bj_cnt);
@@ -523,6 +576,7 @@ int csr_transpose(psfun_csr* a, psfun_csr** out) {
 // y = alpha A x + beta y through the warp-specialised tile pipeline of the
 // persistent kernels (persist.cuh): one block per SM over a contiguous range
 // of tiles, the last warp staging up to four tiles ahead by TMA.
+template <bool ORD>
 __global__ void __launch_bounds__(kSpmvThreads) k_spmv_axpby(CsrDev A, const double* x, double alpha, double beta,
                                                              double* y, int* err, int tiles_per_cta) {
   extern __shared__ __align__(128) unsigned char lz_smem_raw[];
@@ -537,7 +591,7 @@ __global__ void __launch_bounds__(kSpmvThreads) k_spmv_axpby(CsrDev A, const dou
     if (!pipe_produce(A, t0, t0 + min(kLzStages, t1 - t0), sm, pc.issued, stream)) atomicOr(err, DEVERR_TIMEOUT);
   }
   EpiAxpby epi{alpha, beta, y};
-  pipe_spmv(A, x, t0, t1, sm, epi, err, pc, false, stream);
+  pipe_spmv<ORD>(A, x, t0, t1, sm, epi, err, pc, false, stream);
 }
 
 int spmv_device(psfun_csr* a, double alpha, const double* x, double beta, double* y) {
@@ -546,10 +600,13 @@ int spmv_device(psfun_csr* a, double alpha, const double* x, double beta, double
   cudaStream_t s = stream();
   PSF_CUDA(cudaMemsetAsync(errbuf.ptr, 0, sizeof(int), s));
   if (a->ntiles > 0) {
-    static const int gmax = persist_grid_for(k_spmv_axpby);
+    static const int gmax = std::min(persist_grid_for(k_spmv_axpby<false>), persist_grid_for(k_spmv_axpby<true>));
     const int tpc = std::max(1, (a->ntiles + gmax - 1) / gmax);
     const int g = std::max(1, (a->ntiles + tpc - 1) / tpc);
-    k_spmv_axpby<<<g, kSpmvThreads, kLzSmemBytes, s>>>(a->dev(), x, alpha, beta, y, errbuf.as<int>(), tpc);
+    if (a->order)
+      k_spmv_axpby<true><<<g, kSpmvThreads, kLzSmemBytes, s>>>(a->dev(), x, alpha, beta, y, errbuf.as<int>(), tpc);
+    else
+      k_spmv_axpby<false><<<g, kSpmvThreads, kLzSmemBytes, s>>>(a->dev(), x, alpha, beta, y, errbuf.as<int>(), tpc);
     count_launch();
     PSF_CUDA(cudaGetLastError());
   }

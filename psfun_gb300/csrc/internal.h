@@ -103,6 +103,7 @@ struct psfun_csr {
   double norm_inf = 0.0;
   double* diag_inv = nullptr;  // Jacobi preconditioner (lazy)
   unsigned* sched = nullptr;   // SpMV tile work counter + blocks-done counter (zero between launches)
+  uint16_t* order = nullptr;   // skewed row lengths: the rows of every tile by descending length
   int2* tile_desc = nullptr;   // per tile {first row, first stored entry}, ntiles + 1 entries
   int32_t max_tile_rows = 0;
   int32_t max_row = 0;         // longest row (stored entries)
@@ -130,6 +131,7 @@ struct psfun_csr {
     d.n = n; d.nnz = nnz; d.irp = irp; d.ja = ja; d.val = val; d.tile_row = tile_row; d.ntiles = ntiles;
     d.sched = sched;
     d.tile_desc = tile_desc;
+    d.order = order;
     d.stream = (nnz * 12 + n * 4) > ((int64_t)64 << 20) ? 1 : 0;
     return d;
   }

@@ -118,8 +118,10 @@ PSF_DEVINL bool pipe_produce(const CsrDev& A, int tb, int te, LzSmem& sm, unsign
 // SpMV over the CTA's tiles [t0, t1) through the pipeline; epi(r, sum) is
 // called once per row by one thread (its accumulators stay with that thread).
 // prefetch_next: stage the first tiles of the same range again for the next
-// pass.  Returns false on timeout.
-template <class Epi>
+// pass.  Returns false on timeout.  ORD: with the rows of a tile taken in
+// A.order (in the plain product; in the Lanczos step the second form of the
+// row loop costs grid stencils 1.5%).
+template <bool ORD = false, class Epi>
 PSF_DEVINL bool pipe_spmv(const CsrDev& A, const double* __restrict__ x, int t0, int t1, LzSmem& sm, Epi& epi,
                           int* err, PipeCounters& pc, bool prefetch_next, bool stream) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -133,7 +135,7 @@ PSF_DEVINL bool pipe_spmv(const CsrDev& A, const double* __restrict__ x, int t0,
     }
     return ok;
   }
-  const int ctid = threadIdx.x;  // 0 .. kConsumerWarps*32-1
+  static_assert(kTileRows == kConsumerWarps * 32, "32 rows per consumer warp and tile");
   for (int t = t0; t < t1; ++t) {
     const unsigned b = pc.consumed % kLzStages;
     if (!mbar_wait(&sm.bar[b], (pc.consumed / kLzStages) & 1u)) {
@@ -152,7 +154,15 @@ PSF_DEVINL bool pipe_spmv(const CsrDev& A, const double* __restrict__ x, int t0,
     } else {
       const SpmvTile& tb = sm.buf[b];
       const int nr = ti.r1 - ti.r0;
-      for (int base = ctid & ~31; base < nr; base += kConsumerWarps * 32) spmv_rows32(tb, ti, base, x, epi);
+      if (ORD) {
+        const int base = 32 * (int)((unsigned)(warp + t) % (unsigned)kConsumerWarps);
+        if (base < nr) {
+          const int o = base + lane;
+          spmv_rows32<true>(tb, ti, o < nr ? tb.order[o + (ti.r0 & 7)] : nr, x, epi);
+        }
+      } else if (warp * 32 < nr) {
+        spmv_rows32<false>(tb, ti, warp * 32 + lane, x, epi);
+      }
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(&sm.empty[b]);
