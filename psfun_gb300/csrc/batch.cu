@@ -607,7 +607,7 @@ PSF_DEVINL void final_quad(const BInst& I, const BatchArgs& B) {
     if (r < m) h = al[r + 1] * g[r];
     if (r >= 1) h = fma(be[r + 1], g[r - 1], h);
     if (r + 1 < m) h = fma(be[r + 2], g[r + 1], h);
-    pa(I, q, PA_COEF, nl)[r] = I.eta * h * pa(I, q, PA_S, nl)[r + 1];
+    pa(I, q, PA_COEF, nl)[r] = (h == 0.0) ? 0.0 : I.eta * h * pa(I, q, PA_S, nl)[r + 1];  // s infinite: exact breakdown
   }
   __syncthreads();
   if (threadIdx.x < R) {
@@ -809,7 +809,7 @@ PSF_DEVINL void warp_estimate(const BInst& I, int i, const BatchArgs& B, zc* scr
 // converges meanwhile stops a step or two later, which changes nothing that
 // its result uses (later basis slots and entries of T), and the first
 // converged iteration is the one taken, as in the serial order.  On the
-// finalising block an estimate of order 17 costs ~100 us between two grid
+// finalising block an estimate of order 18 costs ~40 us between two grid
 // barriers, with every other SM waiting; 24 uneven graphs (2-65 thousand
 // rows, 4 right-hand sides): 7.60 -> 4.87 ms with the cheaper
 // phases below, 7.0 by the monitors alone.

@@ -2191,7 +2191,7 @@ __global__ void __launch_bounds__(kDenseThreads) k_ms_final(KState st, MsParams 
     if (r < m) h = HAT(st, r + 1, r + 1) * g[r];
     if (r >= 1) h = fma(HAT(st, r + 1, r), g[r - 1], h);
     if (r + 1 < m) h = fma(HAT(st, r + 1, r + 2), g[r + 1], h);
-    st.coef[r] = mp.eta * h * st.s[r + 1];
+    st.coef[r] = (h == 0.0) ? 0.0 : mp.eta * h * st.s[r + 1];  // s is infinite past an exact breakdown
   }
   __syncthreads();
   if (threadIdx.x == 0) {
