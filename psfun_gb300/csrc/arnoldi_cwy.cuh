@@ -32,14 +32,11 @@
 // grid on the integer pipe (fixsum.cuh).
 #pragma once
 
-struct CwyPlan {
-  int G = 0;  // blocks that run the steps (0: no plan)
-  int chunk = 0, rt = 1, threads = 0;
+struct CwyPlan : CwyShape {
   bool vs = false;
   size_t smem = 0;
 };
 
-constexpr int kCwyMaxThreads = 640;
 constexpr int kCwyMaxNl = 128;
 constexpr size_t kCwySmemMax = 220 * 1024;  // leaves the estimate monitors' static shared memory
 
@@ -118,7 +115,7 @@ PSF_DEVINL bool cwy_dots(const CwyDots& d, const double* v1, int64_t ldk, int kq
 }
 
 template <bool VS>
-__global__ void __launch_bounds__(kCwyMaxThreads, 1) k_ar_cwy(KState st, CsrDev A, double scaling, int chunk, int rt,
+__global__ void __launch_bounds__(kCwyThreads, 1) k_ar_cwy(KState st, CsrDev A, double scaling, int chunk, int rt,
                                                               int ew, int monitors, long long* acc_all, double* Lg,
                                                               LzMonitor mon) {
   extern __shared__ __align__(16) double cwy_sm[];
@@ -229,8 +226,11 @@ __global__ void __launch_bounds__(kCwyMaxThreads, 1) k_ar_cwy(KState st, CsrDev 
           case 3: ok = cwy_dots<VS, 3>(d, v1, ldk, kq, kg); break;
           case 4: ok = cwy_dots<VS, 4>(d, v1, ldk, kq, kg); break;
           case 5: ok = cwy_dots<VS, 5>(d, v1, ldk, kq, kg); break;
-          default: ok = cwy_dots<VS, 6>(d, v1, ldk, kq, kg); break;
+          case 6: ok = cwy_dots<VS, 6>(d, v1, ldk, kq, kg); break;
+          case 7: ok = cwy_dots<VS, 7>(d, v1, ldk, kq, kg); break;
+          default: ok = false;  // no plan has more (kCwyMaxRt)
         }
+        static_assert(kCwyMaxRt == 7, "one case per row count of a plan");
         if (!ok) s_bad = 1;
       }
       __syncthreads();
@@ -381,19 +381,13 @@ __global__ void __launch_bounds__(kCwyMaxThreads, 1) k_ar_cwy(KState st, CsrDev 
 
 // Grid, rows per block and shared memory of k_ar_cwy, or none: Krylov
 // dimension above kCwyMaxNl, a row above 64 entries (one thread per row), n of
-// 2^19 rows and more, or monitors that do not fit beside it.
+// 2^19 rows and more, no shape (cwy_shape), or monitors that do not fit beside
+// it.
 static CwyPlan cwy_plan(int64_t n, int nl, int max_row, int monitors, size_t min_smem) {
   CwyPlan p;
   if (nl > kCwyMaxNl || max_row > 64 || n >= ((int64_t)1 << 19) || n < 1) return p;
-  const int maxG = sm_count() - monitors;
-  if (maxG < 1) return p;
-  p.G = (int)std::max<int64_t>(1, std::min<int64_t>(maxG, (n + 63) / 64));
-  p.chunk = (int)((n + p.G - 1) / p.G);
-  p.chunk = (p.chunk + 1) & ~1;
-  p.G = (int)((n + p.chunk - 1) / p.chunk);
-  p.rt = (p.chunk + kCwyMaxThreads - 1) / kCwyMaxThreads;
-  const int nrg = (p.chunk + 32 * p.rt - 1) / (32 * p.rt);
-  p.threads = 32 * (nrg >= 16 ? nrg : nrg * (16 / nrg));
+  static_cast<CwyShape&>(p) = cwy_shape(n, sm_count() - monitors);
+  if (p.G == 0) return CwyPlan();
   p.vs = cwy_smem_bytes(nl, p.chunk, p.rt, true) <= kCwySmemMax;
   p.smem = std::max(cwy_smem_bytes(nl, p.chunk, p.rt, p.vs), min_smem);
   const void* kern = p.vs ? (const void*)k_ar_cwy<true> : (const void*)k_ar_cwy<false>;

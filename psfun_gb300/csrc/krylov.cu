@@ -27,6 +27,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "cwy_shape.h"
 #include "fixsum.cuh"
 #include "internal.h"
 #include "persist.cuh"
