@@ -1462,6 +1462,13 @@ static int lz_norm_exponent(double norm_inf, int64_t n) {
   return bound > 0.0 ? (std::isfinite(bound) ? std::ilogb(bound) + 1 : 1000) : 0;
 }
 
+// ||w|| <= |scaling| ||A||_2 ||v||, ||A||_2 <= sqrt(n) ||A||_inf; 2^ew bounds it
+// with a bit to spare.
+static int cwy_norm_exponent(double scaling, double norm_inf, int64_t n) {
+  const double bound = std::fabs(scaling) * norm_inf * std::sqrt((double)n);
+  return bound > 0.0 ? (std::isfinite(bound) ? std::ilogb(bound) + 2 : 1000) : 0;
+}
+
 // Steps [i_begin, i_end) in one cooperative launch; with a monitor the grid
 // holds the compute CTAs and the monitor block.
 template <int MODE>
@@ -1791,9 +1798,7 @@ int krylov_apply_device(psfun_krylov* meth, psfun_serial* fun, psfun_csr* a, dou
     mon.scr_stride = lz_scr_stride;
     mon.count = kCwyMonitors;
     double sc = scaling;
-    // ||w|| <= |scaling| ||A||_2 ||v||, ||A||_2 <= sqrt(n) ||A||_inf; 2^ew bounds it with a bit to spare
-    const double bound = std::fabs(scaling) * a->norm_inf * std::sqrt((double)n);
-    int ew = bound > 0.0 ? (std::isfinite(bound) ? std::ilogb(bound) + 2 : 1000) : 0;
+    int ew = cwy_norm_exponent(scaling, a->norm_inf, n);
     int monitors = istop == 1 ? kCwyMonitors : 0;
     int chunk = cwy.chunk, rt = cwy.rt;
     long long* acc = reinterpret_cast<long long*>(st.coef + (ldh + 2));
@@ -1812,19 +1817,30 @@ int krylov_apply_device(psfun_krylov* meth, psfun_serial* fun, psfun_csr* a, dou
   };
   if ((istop == 2 || lz_mon || ar_mon) && !userf && !prof_enabled() && !sai) {
     // fixed-length solve: one CUDA graph, captured once per launch key
-    // the device arrays of the matrix are part of the key: a handle can be
-    // destroyed and another created at the same address
+    // everything that the launches carry is part of the key: a handle can be
+    // destroyed and another created at the same address, with the same device
+    // arrays, and the buffers of the method can move
     struct Key {
-      const void* a; const void* x; void* y; const void* V; int64_t n; int nl, arnoldi, keeplast, gs, gv, gm;
+      KState st;  // no padding: two 64-bit and two 32-bit sizes, then pointers
+      const void* a; const void* x; void* y; int arnoldi, keeplast, gs, gv, gm;
       FunParams fp; double scaling;
-      const void *irp, *ja, *val, *tiles, *par;
+      const void *irp, *ja, *val, *tiles, *tile_row, *order, *sched, *par, *dgroup;
+      int64_t nnz; int ntiles, stream, max_row, ea, ew;
       int istop; double eps;
+      CwyPlan cwy;
     } key;
-    memset(&key, 0, sizeof key);
-    key.istop = istop; key.eps = eps; key.par = (lz_mon || ar_mon) ? meth->par.ptr : nullptr;
-    key.irp = A.irp; key.ja = A.ja; key.val = A.val; key.tiles = A.tile_desc;
-    key.a = a; key.x = x; key.y = y; key.V = st.V; key.n = n; key.nl = nl; key.arnoldi = arnoldi;
+    memset((void*)&key, 0, sizeof key);
+    key.st = st; key.istop = istop; key.eps = eps; key.par = (lz_mon || ar_mon) ? meth->par.ptr : nullptr;
+    key.dgroup = meth->dgroup.ptr;
+    key.irp = A.irp; key.ja = A.ja; key.val = A.val; key.tiles = A.tile_desc; key.tile_row = A.tile_row;
+    key.order = A.order; key.sched = A.sched; key.nnz = A.nnz; key.ntiles = A.ntiles; key.stream = A.stream;
+    // the windows of the sums follow the norm of the matrix
+    key.max_row = a->max_row; key.ea = lz_norm_exponent(a->norm_inf, n);
+    key.ew = cwy_norm_exponent(scaling, a->norm_inf, n);
+    key.a = a; key.x = x; key.y = y; key.arnoldi = arnoldi;
     key.keeplast = meth->keeplast; key.gs = gs; key.gv = gv; key.gm = gm; key.fp = fpk; key.scaling = scaling;
+    key.cwy.G = cwy.G; key.cwy.chunk = cwy.chunk; key.cwy.rt = cwy.rt; key.cwy.threads = cwy.threads;
+    key.cwy.vs = cwy.vs; key.cwy.smem = cwy.smem;
     const unsigned char* kb = reinterpret_cast<const unsigned char*>(&key);
     std::vector<unsigned char> kv(kb, kb + sizeof key);
     if (!meth->graph || meth->graph_key != kv) {
