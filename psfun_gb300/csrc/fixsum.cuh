@@ -11,11 +11,12 @@
 // four redux.sync, over a block and over the grid as two 64-bit limbs.
 //
 // The window holds every addend above 2^(E-43) exactly and cuts the others at
-// 2^(E-96), so the sum is exact to 2^(E-96) per addend, whatever their number:
-// more accurate than any FP64 order of additions, and the same bits for every
-// order, which lets the blocks of a grid add into one pair of words with
+// 2^(E-96), so the sum is exact to 2^(E-96) per addend, whatever their number
+// and order, which lets the blocks of a grid add into one pair of words with
 // atomics instead of publishing partials that every block has to read back and
-// add up.  An addend outside the window (Inf, NaN, or a bound that does not
+// add up.  That is more accurate than FP64 additions while the sum's largest
+// addends are near the bound, and less where all of them are far below it: the
+// callers look at how far.  An addend outside the window (Inf, NaN, or a bound that does not
 // hold) is reported by the return value; the callers turn the sum into NaN.
 #pragma once
 
@@ -131,17 +132,13 @@ PSF_DEVINL bool fix192_limbs(double p, int E, long long (&w)[4]) {
   return ok;
 }
 
-PSF_DEVINL double fix192_value(long long w3, long long w2, long long w1, long long w0, int E) {
-  w1 += w0 >> 48;
-  w0 &= kFixMask48;
-  w2 += w1 >> 48;
-  w1 &= kFixMask48;
-  w3 += w2 >> 48;
-  w2 &= kFixMask48;
-  const double c = 281474976710656.0;  // 2^48
-  const double v = fma(fma(fma((double)w3, c, (double)w2), c, (double)w1), c, (double)w0);
-  return scale_pow2(v, E - 192);
+// A non-zero addend with a mantissa bit below a window's unit 2^U.
+PSF_DEVINL bool fix_cut(double p, int U) {
+  const unsigned hi = (unsigned)__double2hiint(p) & 0x7fffffffu;
+  return (hi | (unsigned)__double2loint(p)) != 0u && max((int)(hi >> 20), 1) - 1075 < U;
 }
+// |p| < 2^E (Inf and NaN are not).
+PSF_DEVINL bool fix_below(double p, int E) { return (int)((__double2hiint(p) >> 20) & 0x7ff) - 1022 <= min(E, 1024); }
 
 // ---------------------------------------------------------------------------
 // Grid sums whose words count their own arrivals.  Each block adds to every
@@ -151,42 +148,59 @@ PSF_DEVINL double fix192_value(long long w3, long long w2, long long w1, long lo
 // the last block, where a counter barrier, the fetch of every block's partial
 // and their FP64 butterfly took 5500-6500 clocks (152 blocks; polling one slot
 // per block instead of one word per limb is no cure: 152 x 152 polls made the
-// same reduction 3000 clocks slower).  G <= 200; a block whose addend does not
-// fit the window marks the top limb, and the sum becomes NaN: the bound E
-// passed to it lies 3 bits above what the sum can reach, which keeps unmarked
-// top limbs below 2^46.
+// same reduction 3000 clocks slower).  G <= 200.  The words start at
+// count_start, whose bias keeps the sums of the limbs positive, so that the
+// arrivals are the top byte as it is.
+//
+// The window is placed by a bound that the sum may stay far below (or, where
+// the bound does not hold, lie above), so the sum itself says whether it
+// stands.  The top word has, above a 40-bit limb, two more 8-bit counts: of
+// the blocks whose addend has bits below the window's unit (bits 40-47), and
+// of those whose addend is not below 2^(E-17) (bits 48-55; the others' top
+// limbs are at most 2^31, and 200 of them below 2^39).  Each cut addend is off
+// by less than one unit, so a total of 2^62 units or more is off by less than
+// 2^-54 of itself, and one without cut addends is exact.  Otherwise the reader
+// has to sum in FP64.
 // ---------------------------------------------------------------------------
 constexpr int kCountMaxBlocks = 200;
 constexpr long long kCountOne = 1ll << 56;
-constexpr long long kCountMark = 1ll << 47;
+constexpr long long kCountBad = 1ll << 48;
+constexpr long long kCountCut = 1ll << 40;
+constexpr int kCountHeadBits = 17;  // of the top limb's 48, above an addend
+constexpr long long kCountLowBias = 1ll << 55, kCountTopBias = 1ll << 39;
 
+// What word q of N starts at.
+__host__ __device__ constexpr long long count_start(int q, int N) {
+  return q + 1 < N ? kCountLowBias : kCountTopBias;
+}
+
+// ok: the addend is below 2^(E-17); cut: it has bits below the unit.
 template <int N>
-PSF_DEVINL void count_post(long long* words, long long (&w)[N], bool ok) {
+PSF_DEVINL void count_post(long long* words, long long (&w)[N], bool ok, bool cut) {
 #pragma unroll
   for (int q = 0; q + 1 < N; ++q) {  // limbs into [-2^47, 2^47)
     const long long carry = (w[q] + (1ll << 47)) >> 48;
     w[q] -= carry << 48;
     w[q + 1] += carry;
   }
-  if (!ok) w[N - 1] = kCountMark;
+  const long long flag = cut ? kCountOne + kCountCut : kCountOne;
 #pragma unroll
-  for (int q = 0; q < N; ++q) red_add_s64(words + q, w[q] + kCountOne);
+  for (int q = 0; q + 1 < N; ++q) red_add_s64(words + q, w[q] + kCountOne);
+  red_add_s64(words + N - 1, ok ? w[N - 1] + flag : kCountOne + kCountBad);
 }
 
-// One thread: waits (bounded) for G arrivals on each word; w the sums.
+// One thread: waits (bounded) for G arrivals on each word; the sum in units of
+// the window, and whether it stands.
 template <int N>
-PSF_DEVINL bool count_wait(const long long* words, int G, long long (&w)[N], bool& ok, int* err) {
+PSF_DEVINL bool count_wait(const long long* words, int G, double& units, bool& stands, int* err) {
+  long long w[N];
   unsigned long long t0 = 0;
   for (unsigned n = 0;; ++n) {
     bool all = true;
 #pragma unroll
     for (int q = 0; q < N; ++q) w[q] = ld_relaxed_s64(words + q);
 #pragma unroll
-    for (int q = 0; q < N; ++q) {
-      const long long c = (long long)((unsigned long long)(w[q] + (1ll << 55)) >> 56);
-      all &= c == G;
-      w[q] -= (long long)((unsigned long long)c << 56);
-    }
+    for (int q = 0; q < N; ++q) all &= (int)((unsigned long long)w[q] >> 56) == G;
     if (all) break;
     if ((n & 63u) == 63u) {
       if (t0 == 0) t0 = globaltimer_ns();
@@ -197,8 +211,54 @@ PSF_DEVINL bool count_wait(const long long* words, int G, long long (&w)[N], boo
       }
     }
   }
-  ok = w[N - 1] < (1ll << 46) && w[N - 1] > -(1ll << 46);
+  const unsigned flags = (unsigned)((unsigned long long)w[N - 1] >> 40) & 0xffffu;
+#pragma unroll
+  for (int q = 0; q + 1 < N; ++q) w[q] = (w[q] & (kCountOne - 1)) - kCountLowBias;
+  w[N - 1] = (w[N - 1] & (kCountCut - 1)) - kCountTopBias;
+#pragma unroll
+  for (int q = 0; q + 1 < N; ++q) {
+    w[q + 1] += w[q] >> 48;
+    w[q] &= kFixMask48;
+  }
+  units = (double)w[N - 1];
+#pragma unroll
+  for (int q = N - 2; q >= 0; --q) units = fma(units, 281474976710656.0, (double)w[q]);  // 2^48
+  stands = flags == 0u;
+  if (!stands) stands = flags < 0x100u && fabs(units) >= 4611686018427387904.0;  // no bad addend, 2^62
   return true;
+}
+
+// The same sum in FP64, by one warp of every block: the partials of all blocks
+// in `part`, their arrivals counted in *arrivals (zero before), the total (a
+// fixed order) in *out, in shared memory.  False when the wait gave up.
+static __device__ __noinline__ bool count_sum_fp64(double mine, double* part, long long* arrivals, int bid, int G,
+                                                   int* err, double* out) {
+  const int lane = threadIdx.x & 31;
+  int ok = 1;
+  if (lane == 0) {
+    *(volatile double*)(part + bid) = mine;
+    __threadfence();
+    red_add_s64(arrivals, 1);
+    const unsigned long long t0 = globaltimer_ns();
+    while (ld_relaxed_s64(arrivals) < G) {
+      if (*(volatile int*)err != 0) { ok = 0; break; }
+      if (globaltimer_ns() - t0 > kWaitLimitNs) {
+        atomicOr(err, DEVERR_TIMEOUT);
+        ok = 0;
+        break;
+      }
+      __nanosleep(32);
+    }
+    __threadfence();
+  }
+  __syncwarp();
+  ok = __shfl_sync(0xffffffffu, ok, 0);
+  double v = 0.0;
+  if (ok)
+    for (int b = lane; b < G; b += 32) v += *(const volatile double*)(part + b);
+  v = warp_sum(v);
+  if (lane == 0) *out = v;
+  return ok != 0;
 }
 
 }  // namespace psf

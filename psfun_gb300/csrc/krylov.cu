@@ -65,9 +65,13 @@ constexpr int kDenseThreads = 256;
 constexpr int kMgsThreads = 1024;
 // The words of the Lanczos reductions (fixsum.cuh) in KState::partials (2 x 4096
 // doubles): three buffers that the steps use in turn, each the two limbs of
-// alpha, CTA 0's answer to a stop request and the four limbs of the norm on a
-// 64-byte line.
-constexpr int kLzWordsAt = 4096, kLzBuf = 8, kLzWords = 3 * kLzBuf;
+// alpha (0), CTA 0's answer to a stop request (2) and the four limbs of the
+// norm (4) on a 64-byte line, then the arrivals of the FP64 sums of alpha (8)
+// and of the norm (9).
+constexpr int kLzWordsAt = 4096, kLzBuf = 16, kLzUsed = 10, kLzWords = 3 * kLzBuf;
+__host__ __device__ constexpr long long lz_word_start(int q) {
+  return q < 2 ? count_start(q, 2) : q >= 4 && q < 8 ? count_start(q - 4, 4) : 0;
+}
 
 // ---------------------------------------------------------------------------
 // kernels
@@ -94,8 +98,9 @@ __global__ void __launch_bounds__(kVecThreads) k_init(KState st, const double* _
   __shared__ double red[32];
   double* w1 = WAT(st, 1);
   double acc = 0.0;
-  // the sums of the Lanczos reductions start at zero
-  if (blockIdx.x == 0 && threadIdx.x < kLzWords) st.partials[kLzWordsAt + threadIdx.x] = 0.0;
+  // the words of the Lanczos reductions
+  if (blockIdx.x == 0 && threadIdx.x < kLzWords)
+    reinterpret_cast<long long*>(st.partials)[kLzWordsAt + threadIdx.x] = lz_word_start(threadIdx.x % kLzBuf);
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < st.n; r += (int64_t)gridDim.x * blockDim.x) {
     const double v = x[r];
     w1[r] = v;
@@ -122,16 +127,21 @@ __global__ void __launch_bounds__(kVecThreads) k_init(KState st, const double* _
 // Each CTA owns a contiguous range of row tiles (static schedule: the tile
 // after next is staged by TMA while the current one is computed).  Per step:
 //   phase 1  u = A W_i on the CTA's rows, partial W_i . u
-//   reduce   every CTA sums the partials in the same order -> alpha_i (no
-//            fence: phase 2 touches the CTA's own rows only)
+//   reduce   every CTA posts its partial's limbs and reads the completed words
+//            -> alpha_i (no fence: phase 2 touches the CTA's own rows only)
 //   phase 2  W_{i+1} = 2^k (u - alpha W_i - c2 W_{i-1}), partial ||.||^2
-//   reduce   every CTA sums -> beta_{i+1}, s_{i+1}; with fences, as the next
-//            SpMV reads W_{i+1} of other CTAs
+//   reduce   the same -> beta_{i+1}, s_{i+1}; with fences, as the next SpMV
+//            reads W_{i+1} of other CTAs
 // (fixed-point sums that count their arrivals, fixsum.cuh).  Every CTA derives
 // the scalars itself, so none is re-read from memory, and CTA 0 records H, s
-// and itx for the estimate / final kernels.  The bounds of the sums come from
-// ||A||_2 <= 2^ea: |W.u| <= 2^ea ||W||^2, and ||w|| <= 5 2^ea ||W|| as c2 W_{i-1}
-// is the previous step's ||w|| long; ||W|| = 1 / s_i.  Measured:
+// and itx for the estimate / final kernels.  The windows of the sums come from
+// ||A||_2 <= ||A||_inf < 2^ea for a symmetric A: |W.u| <= 2^ea ||W||^2, and
+// ||w|| <= 5 2^ea ||W|| as c2 W_{i-1} is the previous step's ||w|| long;
+// ||W|| = 1 / s_i.  A unit of alpha is then 2^(ea-78), one of beta^2
+// 2^(2 ea-168) (unit vectors).  Sums far below the bound that have lost bits
+// (alpha below 2^(ea-16), beta below 2^(ea-53): vectors that do not meet the
+// rows of the norm), or above it (A not symmetric), are taken again in FP64
+// from the CTAs' partials (count_sum_fp64), by all CTAs alike.  Measured:
 // 100 x 100, istop 1: 0.321 -> 0.298 ms; multi-shift on 96^3, 438 steps: 15.03 ->
 // 14.61.
 // ---------------------------------------------------------------------------
@@ -299,23 +309,23 @@ PSF_DEVINL void lz_persist_body(KState& st, const CsrDev& A, int i_begin, int i_
     }
     long long* const acc_w = words + (i % 3) * kLzBuf;
     {
-      double S = 0.0, stop = 0.0;
+      double S = 0.0;
       block_sum_store_512(acc, sm.vals, sm.red, &S);
-      bool up = true;
+      bool up = true, stands = true;
       if (threadIdx.x == 0) {
         sc = sm.scal[0];
-        const int E = ea - 2 * ilog2_normal(sc) + 4;
+        const int E = ea - 2 * ilog2_normal(sc) + 1 + kCountHeadBits;
         long long w[2];
-        bool ok;
         {
           int b[4];
-          ok = fix96_pieces(S, E, b);
+          fix96_pieces(S, E, b);
           w[0] = (long long)b[0] + ((long long)b[1] << 24);
           w[1] = (long long)b[2] + ((long long)b[3] << 24);
         }
-        count_post(acc_w, w, ok);
+        count_post(acc_w, w, fix_below(S, E - kCountHeadBits), fix_cut(S, E - 96));
+        double sum = 0.0, stop = 0.0;
+        up = count_wait<2>(acc_w, G, sum, stands, &c->err);
         if (kMon) {  // CTA 0's answer has long been there when the sum completes
-          up = count_wait(acc_w, G, w, ok, &c->err);
           long long d;
           const unsigned long long t0 = globaltimer_ns();
           while (up && ((d = *(volatile long long*)(acc_w + 2)) >> 1) != i) {
@@ -325,25 +335,35 @@ PSF_DEVINL void lz_persist_body(KState& st, const CsrDev& A, int i_begin, int i_
             }
           }
           stop = up && (d & 1) ? 1.0 : 0.0;
-        } else {
-          up = count_wait(acc_w, G, w, ok, &c->err);
         }
-        S = ok ? fix96_value(w[1], w[0], E) : __longlong_as_double(0x7ff8000000000000ll);
-        const double a = sc * sc * S;
+        const double a = sc * sc * scale_pow2(sum, E - 96);
         sm.scal[2] = a;
         sm.scal[4] = stop;
-        // the next step's words start at zero: every CTA has read what they
-        // held two steps ago, and adds to them after this CTA's next post
+        sm.scal[6] = up ? 0.0 : 1.0;
+        // the next step's words: every CTA has read what they held two steps
+        // ago, and adds to them after this CTA's next post
         if (bid == 0)
-          for (int q = 0; q < kLzBuf; ++q) words[((i + 1) % 3) * kLzBuf + q] = 0;
+#pragma unroll
+          for (int q = 0; q < kLzUsed; ++q) words[((i + 1) % 3) * kLzBuf + q] = lz_word_start(q);
         if (bid == 0 && stop == 0.0) {
           HAT(st, i, i) = a;
           if (i >= 2) c->itx = i - 1;
         }
       }
-      if (__syncthreads_or(!up)) {
-        drain(i - i_begin + 1);
-        return;
+      if (__syncthreads_or(!up || !stands)) {
+        bool ok = sm.scal[6] == 0.0;
+        if (ok && threadIdx.x < 32) {
+          ok = count_sum_fp64(S, st.partials, acc_w + 8, bid, G, &c->err, &sm.scal[7]);
+          if (threadIdx.x == 0) {
+            const double a = sc * sc * sm.scal[7];
+            sm.scal[2] = a;
+            if (bid == 0 && sm.scal[4] == 0.0) HAT(st, i, i) = a;
+          }
+        }
+        if (__syncthreads_or(!ok)) {
+          drain(i - i_begin + 1);
+          return;
+        }
       }
     }
     if (kMon && sm.scal[4] != 0.0) {  // the monitor has decided: leave before the update
@@ -385,17 +405,9 @@ PSF_DEVINL void lz_persist_body(KState& st, const CsrDev& A, int i_begin, int i_
     {
       double S = 0.0;
       block_sum_store_512(acc2, sm.vals, sm.red, &S);
-      bool up = true;
-      if (threadIdx.x == 0) {
-        const int E = 2 * (ea - k2 + 3) + 4;
-        long long w[4];
-        bool ok = fix192_limbs(S, E, w);
-        __threadfence();  // the block's rows of W_{i+1}, ordered before by block_sum_store_512's barriers
-        count_post(acc_w + 4, w, ok);
-        up = count_wait(acc_w + 4, G, w, ok, &c->err);
-        __threadfence();
-        S = ok ? fix192_value(w[3], w[2], w[1], w[0], E) : __longlong_as_double(0x7ff8000000000000ll);
-        const double wn = sqrt(S);
+      bool up = true, stands = true;
+      auto finish = [&](double sum) {  // thread 0
+        const double wn = sqrt(sum);
         const double bt = sc * wn;
         sm.scal[3] = bt;
         sm.scal[5] = wn;
@@ -412,10 +424,29 @@ PSF_DEVINL void lz_persist_body(KState& st, const CsrDev& A, int i_begin, int i_
             st_release_gpu(&c->pub, i);
           }
         }
+      };
+      if (threadIdx.x == 0) {
+        const int E = 2 * (ea - k2 + 3) + 1 + kCountHeadBits;
+        long long w[4];
+        fix192_limbs(S, E, w);
+        double sum = 0.0;
+        __threadfence();  // the block's rows of W_{i+1}, ordered before by block_sum_store_512's barriers
+        count_post(acc_w + 4, w, fix_below(S, E - kCountHeadBits), fix_cut(S, E - 192));
+        up = count_wait<4>(acc_w + 4, G, sum, stands, &c->err);
+        __threadfence();
+        sm.scal[6] = up ? 0.0 : 1.0;
+        if (up && stands) finish(scale_pow2(sum, E - 192));
       }
-      if (__syncthreads_or(!up)) {
-        drain(i - i_begin + 1);
-        return;
+      if (__syncthreads_or(!up || !stands)) {
+        bool ok = sm.scal[6] == 0.0;
+        if (ok && threadIdx.x < 32) {
+          ok = count_sum_fp64(S, st.partials + kCountMaxBlocks, acc_w + 9, bid, G, &c->err, &sm.scal[7]);
+          if (ok && threadIdx.x == 0) finish(sm.scal[7]);
+        }
+        if (__syncthreads_or(!ok)) {
+          drain(i - i_begin + 1);
+          return;
+        }
       }
     }
     const double beta = sm.scal[3];
@@ -1455,11 +1486,9 @@ static int persist_grid() {
   return g;
 }
 
-// ||A||_2 <= sqrt(n) ||A||_inf < 2^ea (a symmetric A needs no sqrt(n), but the
-// method does not ask for one).
-static int lz_norm_exponent(double norm_inf, int64_t n) {
-  const double bound = norm_inf * std::sqrt((double)std::max<int64_t>(n, 1));
-  return bound > 0.0 ? (std::isfinite(bound) ? std::ilogb(bound) + 1 : 1000) : 0;
+// ||A||_2 <= ||A||_inf < 2^ea for a symmetric A (see k_lz_persist).
+static int lz_norm_exponent(double norm_inf) {
+  return norm_inf > 0.0 ? (std::isfinite(norm_inf) ? std::ilogb(norm_inf) + 1 : 1000) : 0;
 }
 
 // ||w|| <= |scaling| ||A||_2 ||v||, ||A||_2 <= sqrt(n) ||A||_inf; 2^ew bounds it
@@ -1486,7 +1515,7 @@ static int launch_lz_persist_mode(KState& st, const CsrDev& A, double norm_inf, 
   G = (A.ntiles + tpc - 1) / tpc;
   if (G < 1) G = 1;
   LzMonitor m = mon;
-  int ea = lz_norm_exponent(norm_inf, st.n);
+  int ea = lz_norm_exponent(norm_inf);
   void* args[] = {(void*)&st, (void*)&A, (void*)&i_begin, (void*)&i_end, (void*)&tpc, (void*)&ea, (void*)&m};
   PSF_CUDA(cudaLaunchCooperativeKernel((void*)k_lz_persist<MODE>, dim3(G + extra), dim3(kSpmvThreads), args,
                                        kLzSmemBytes, s));
@@ -1835,7 +1864,7 @@ int krylov_apply_device(psfun_krylov* meth, psfun_serial* fun, psfun_csr* a, dou
     key.irp = A.irp; key.ja = A.ja; key.val = A.val; key.tiles = A.tile_desc; key.tile_row = A.tile_row;
     key.order = A.order; key.sched = A.sched; key.nnz = A.nnz; key.ntiles = A.ntiles; key.stream = A.stream;
     // the windows of the sums follow the norm of the matrix
-    key.max_row = a->max_row; key.ea = lz_norm_exponent(a->norm_inf, n);
+    key.max_row = a->max_row; key.ea = lz_norm_exponent(a->norm_inf);
     key.ew = cwy_norm_exponent(scaling, a->norm_inf, n);
     key.a = a; key.x = x; key.y = y; key.arnoldi = arnoldi;
     key.keeplast = meth->keeplast; key.gs = gs; key.gv = gv; key.gm = gm; key.fp = fpk; key.scaling = scaling;
@@ -2345,7 +2374,7 @@ static int shifted_pair(psfun_krylov* wx, psfun_krylov* wg, DevBuf& msx, DevBuf&
   const int half = std::min(blocks / 2 - 1, kCountMaxBlocks);
   int tpc = std::max(1, (a->ntiles + half - 1) / half);
   const int G = std::max(1, (a->ntiles + tpc - 1) / tpc);
-  int ea = lz_norm_exponent(a->norm_inf, a->n), i_end = itmax + 1;
+  int ea = lz_norm_exponent(a->norm_inf), i_end = itmax + 1;
   CsrDev A = a->dev();
   LzMonitor mx, mg;
   memset(&mx, 0, sizeof mx);
