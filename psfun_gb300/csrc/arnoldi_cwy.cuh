@@ -30,6 +30,15 @@
 // from L2.  A warp owns 32 rt of the block's rows and every kg-th vector, forms
 // lane partials of the two dots in FP64 and sums them over the lanes and the
 // grid on the integer pipe (fixsum.cuh).
+//
+// The window of V^T w: a lane partial is cut at 2^(ew-96) (unit vectors), so
+// with at most 2^17 of them the coefficients are good to 2^-55 ||w|| while 2^ew
+// is at most 2^24 ||w||.  ||w|| is known one reduction later, from h and beta:
+// ||A|| places only the first step's window, and each step the next one's (12
+// above).  A step whose window turns out wrong (vectors that do not meet the
+// rows of the norm, scales far apart) is run once more, before anything of it
+// is published, with the window from max |w| (an integer maximum over the grid
+// and a barrier of its own).
 #pragma once
 
 struct CwyPlan : CwyShape {
@@ -40,13 +49,20 @@ struct CwyPlan : CwyShape {
 constexpr int kCwyMaxNl = 128;
 constexpr size_t kCwySmemMax = 220 * 1024;  // leaves the estimate monitors' static shared memory
 
-// 64-bit words of one buffer of grid sums: r and l limbs per vector, the three
-// limbs of the norm, the flag.
+// 64-bit words of one buffer of grid sums: r and l limbs per vector, then the
+// four limbs of the norm, and at the offsets below from there the dots outside
+// the window, the high word of max |w| and the norm's addends outside.
 __host__ __device__ inline int cwy_acc_words(int nl) { return 4 * nl + 8; }
+constexpr int kCwyBadDot = 4, kCwyMax = 5, kCwyBadNorm = 6;
+constexpr int kCwyAbove = 24, kCwyNext = 12;  // of a window over log2 ||w||: at most, and for the next step
+// ew and -il[k] (il: floor(log2 s_k), 1 / s_k = ||W_k||) from here up, so that a
+// window's unit, at 2^(ew - il - 96) or 2^(1 - il - il - 96), is never far below
+// the smallest double.
+constexpr int kCwyMinExp = -489;
 
 static size_t cwy_smem_bytes(int nl, int chunk, int rt, bool vs) {
   const size_t nrg = (size_t)(chunk + 32 * rt - 1) / (32 * rt);
-  size_t d = (size_t)chunk * (vs ? nl : 2) + 4 * (size_t)(nl + 2) + 4 * nrg * nl + 3 * 32;
+  size_t d = (size_t)chunk * (vs ? nl : 2) + 4 * (size_t)(nl + 2) + 4 * nrg * nl + 4 * 32;
   return 8 * d + 4 * ((size_t)nl * (nl - 1) / 2 + 2 * (nl + 2)) + 64;
 }
 
@@ -119,7 +135,8 @@ __global__ void __launch_bounds__(kCwyThreads, 1) k_ar_cwy(KState st, CsrDev A, 
                                                               int ew, int monitors, long long* acc_all, double* Lg,
                                                               LzMonitor mon) {
   extern __shared__ __align__(16) double cwy_sm[];
-  __shared__ int s_bad, s_slow, s_end;
+  __shared__ int s_bad, s_slow, s_end, s_wrong, s_ew;
+  __shared__ unsigned s_max[32];  // per warp
   KCtrl* c = st.ctrl;
   const int nl = st.nl, G = gridDim.x - monitors, b = blockIdx.x;
   const int t = threadIdx.x, bd = blockDim.x, lane = t & 31, warp = t >> 5;
@@ -137,35 +154,39 @@ __global__ void __launch_bounds__(kCwyThreads, 1) k_ar_cwy(KState st, CsrDev A, 
   double* lv = rv + nl + 2;                           // l_k
   double* hv = lv + nl + 2;                           // h_k
   long long* part = reinterpret_cast<long long*>(hv + nl + 2);  // [row group][k][r hi, r lo, l hi, l lo]
-  long long* red3 = part + (size_t)4 * nrg * nl;      // [warp][3]
-  float* rf = reinterpret_cast<float*>(red3 + 3 * 32);
-  int* il = reinterpret_cast<int*>(rf + nl + 2);      // floor(log2 s_k)
+  long long* red4 = part + (size_t)4 * nrg * nl;      // [warp][4]
+  float* rf = reinterpret_cast<float*>(red4 + 4 * 32);
+  int* il = reinterpret_cast<int*>(rf + nl + 2);      // floor(log2 s_k), at most -kCwyMinExp
   float* Lf = reinterpret_cast<float*>(il + nl + 2);  // row k (0-based) of L at k (k - 1) / 2
   const int64_t r0 = (int64_t)b * chunk;
   const int nloc = (int)max((int64_t)0, min(r0 + chunk, st.n) - r0);
   const int aw = cwy_acc_words(nl);
   unsigned nb = 0;
   int last = 0;
+  bool pending = false;   // beta of the step before is still to be formed
+  bool measured = false;  // its window came from max |w|
+  bool bad = false;       // a dot of it was outside the window
+  bool measure = false;   // this step is run again
+  int rr = 0;             // steps run, with the repeated ones: three buffers in turn
   const bool zero_x = c->done != 0;
   if (!zero_x) {
     const double* w1 = WAT(st, 1) + r0;
     for (int l = t; l < nloc; l += bd) Vs[l] = w1[l];
     if (t == 0) {
       ss[1] = st.s[1];
-      il[1] = ilog2_normal(ss[1]);
-      s_bad = s_slow = s_end = 0;
+      il[1] = min(ilog2_normal(ss[1]), -kCwyMinExp);
+      s_bad = s_slow = s_end = s_wrong = 0;
+      s_ew = ew;
     }
     __syncthreads();
   }
-  for (int i = 2; i <= nl && !zero_x; ++i) {
+  for (int i = 2; !zero_x; ++i) {
     const int nv = i - 1;
-    long long* acc = acc_all + (size_t)(i % 3) * aw;
-    const double* vl = VS ? Vs + (size_t)(nv - 1) * chunk : Vs;  // rows of W_{i-1}
     // ---- w = scaling s_{i-1} A W_{i-1} on the block's rows (psfun_d_arnoldi.f90:202).
     // s_{i-1} is formed by one thread meanwhile (sqrt and division: ~1200 clocks).
     {
       const double* __restrict__ x = WAT(st, nv);
-      for (int l = t; l < nloc; l += bd) {
+      for (int l = t; l < nloc && i <= nl; l += bd) {
         const int kb = A.irp[r0 + l], ke = A.irp[r0 + l + 1];
         double s = 0.0;
         for (int k = kb; k < ke; k += 4) {
@@ -183,33 +204,78 @@ __global__ void __launch_bounds__(kCwyThreads, 1) k_ar_cwy(KState st, CsrDev A, 
         wl[l] = s;
       }
       if (b == 0 && t == 0) c->stop_dec = *(volatile int*)&c->stop_req;
-      if (i > 2 && lead) {  // the norm of the previous step (every block alike)
-        const long long* pn = acc_all + (size_t)((i - 1) % 3) * aw + 4 * nl;
-        const long long w0 = ld_relaxed_s64(pn), w1 = ld_relaxed_s64(pn + 1), w2 = ld_relaxed_s64(pn + 2);
-        const bool bad = ld_relaxed_s64(pn + 3) != 0;
-        const double beta = bad ? __longlong_as_double(0x7ff8000000000000ll) : sqrt(fix144_value(w2, w1, w0, 2 * ew));
-        const double s = 1.0 / beta;
-        ss[nv] = s;
-        il[nv] = ilog2_normal(s);
-        if (beta == 0.0) s_end = 1;
-        if (b == 0) {
-          HAT(st, nv, nv - 1) = beta;
-          st.s[nv] = s;
-          c->itx = nv - 1;
-          if (beta == 0.0) c->breakdown = 1;
-          if (st.host_flag) st.host_flag[1] = nv;
-          st_release_gpu(&c->pub, nv - 1);
+      if (pending && t >= bd - 32) {  // the norm of the previous step (every block alike)
+        const long long* pn = acc_all + (size_t)((rr + 2) % 3) * aw + 4 * nl;
+        long long w4[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) w4[q] = ld_relaxed_s64(pn + q);
+        const bool badn = ld_relaxed_s64(pn + kCwyBadNorm) != 0;
+        unsigned m = 0u;  // the high word of max |h| orders as the magnitude does
+        for (int k = lane; k < nv - 1; k += 32) m = max(m, (unsigned)__double2hiint(hv[k]) & 0x7fffffffu);
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lead) {
+          const double beta = badn ? __longlong_as_double(0x7ff8000000000000ll)
+                                   : sqrt(scale_pow2(fix_units(w4), 2 * ew + 8 - 192));
+          const int e = (int)(max(m, (unsigned)__double2hiint(beta) & 0x7fffffffu) >> 20) - 1023;  // of ||w||
+          s_wrong = !measured && (bad || badn || ew > max(e + kCwyAbove, kCwyMinExp));
+          if (!s_wrong) {
+            s_ew = e > -1023 ? max(e + kCwyNext, kCwyMinExp) : ew;
+            const double s = 1.0 / beta;
+            if (i <= nl) {
+              ss[nv] = s;
+              il[nv] = min(ilog2_normal(s), -kCwyMinExp);
+            }
+            if (beta == 0.0 && i <= nl) s_end = 1;
+            if (b == 0) {
+              HAT(st, nv, nv - 1) = beta;
+              st.s[nv] = s;
+              c->itx = nv - 1;
+              if (beta == 0.0) c->breakdown = 1;
+              if (st.host_flag) st.host_flag[1] = nv;
+              st_release_gpu(&c->pub, nv - 1);
+            }
+            last = nv - 1;
+          }
         }
-        last = nv - 1;
       }
       __syncthreads();
+      const bool wrong = pending && s_wrong;
+      pending = false;
+      if (wrong) {  // the previous step again
+        if (!VS) {  // its newest vector: this thread's rows
+          for (int l = t; l < nloc; l += bd) Vs[l] = __ldcg(WAT(st, nv - 1) + r0 + l);
+        }
+        i -= 2;
+        measure = true;
+        continue;
+      }
+      if (i > nl) break;
       if (s_end) {  // h(i-1,i-2) == 0: the solve ends on the invariant subspace
         if (b == 0 && t == 0) c->done = 1;
         break;
       }
+      ew = s_ew;
       const double f = scaling * ss[nv];
       for (int l = t; l < nloc; l += bd) wl[l] *= f;
       __syncthreads();
+    }
+    long long* acc = acc_all + (size_t)(rr % 3) * aw;
+    const double* vl = VS ? Vs + (size_t)(nv - 1) * chunk : Vs;  // rows of W_{i-1}
+    if (measure) {
+      unsigned m = 0u;
+      for (int l = t; l < nloc; l += bd) m = max(m, (unsigned)__double2hiint(wl[l]) & 0x7fffffffu);
+      m = __reduce_max_sync(0xffffffffu, m);
+      if (lane == 0) s_max[warp] = m;
+      __syncthreads();
+      if (warp == 0) {
+        m = __reduce_max_sync(0xffffffffu, lane < (bd >> 5) ? s_max[lane] : 0u);
+        if (lane == 0) atomicMax(reinterpret_cast<unsigned*>(acc + 4 * nl + kCwyMax), m);
+      }
+      if (!grid_sync_to(&c->bar_count, (++nb) * (unsigned)G, &c->err)) break;
+      m = (unsigned)ld_relaxed_s64(acc + 4 * nl + kCwyMax);
+      // ||w|| < 2^ew by sqrt(n) and two bits; w of zeros, and one that is not finite, keep what there is
+      if (m > 0u && m < 0x7ff00000u)
+        ew = max((int)(m >> 20) - 1021 + (33 - __clz((unsigned)max((int64_t)1, st.n - 1))) / 2, kCwyMinExp);
     }
     // ---- dots of w and of W_{i-1} with the basis: lane partials over the
     // warp's rows, then the fixed-point sums
@@ -234,44 +300,55 @@ __global__ void __launch_bounds__(kCwyThreads, 1) k_ar_cwy(KState st, CsrDev A, 
         if (!ok) s_bad = 1;
       }
       __syncthreads();
-      if (t < 2 * nv - 1) {  // t < nv: r of vector t + 1; then l of vector t - nv + 1
+      if (t < 2 * nv - 1) {
         const int k = t < nv ? t : t - nv, sel = t < nv ? 0 : 2;
-        long long hi = 0, lo = 0;
+        long long h = 0, l = 0;
         for (int g = 0; g < nrg; ++g) {
           const long long* o = part + ((size_t)g * nl + k) * 4 + sel;
-          hi += o[0];
-          lo += o[1];
+          h += o[0];
+          l += o[1];
         }
-        fix96_carry(hi, lo);
+        fix96_carry(h, l);
         long long* o = acc + (t < nv ? 0 : 2 * nl) + 2 * k;
-        red_add_s64(o, hi);
-        red_add_s64(o + 1, lo);
+        red_add_s64(o, h);
+        red_add_s64(o + 1, l);
       }
-      if (t == 0 && s_bad) red_add_s64(acc + 4 * nl + 3, 1);
+      if (t == bd - 1) {
+        if (s_bad) red_add_s64(acc + 4 * nl + kCwyBadDot, 1);
+        s_bad = 0;
+      }
     }
     if (!grid_sync_to(&c->bar_count, (++nb) * (unsigned)G, &c->err)) break;
-    if (*(volatile int*)&c->stop_dec) {
+    // all words of the step are fetched at once
+    const bool stop = *(volatile int*)&c->stop_dec != 0;
+    const long long bad_word = ld_relaxed_s64(acc + 4 * nl + kCwyBadDot);
+    long long hi = 0, lo = 0;  // thread t < nv: r of vector t + 1; then l of vector t - nv + 1
+    if (t < 2 * nv - 1) {
+      const long long* o = acc + (t < nv ? 2 * t : 2 * nl + 2 * (t - nv));
+      hi = ld_relaxed_s64(o);
+      lo = ld_relaxed_s64(o + 1);
+    }
+    if (stop) {
       if (b == 0 && t == 0) c->done = 1;
       break;
     }
+    bad = bad_word != 0;
     // ---- h = (I + L)^{-1} r
-    const bool bad = ld_relaxed_s64(acc + 4 * nl + 3) != 0;
     if (t < 2 * nv - 1) {
       const bool isr = t < nv;
       const int k = isr ? t : t - nv;
-      const long long* o = acc + (isr ? 0 : 2 * nl) + 2 * k;
-      const long long hi = ld_relaxed_s64(o), lo = ld_relaxed_s64(o + 1);
-      const double sk = ss[k + 1];
-      double v = fix96_value(hi, lo, isr ? ew - il[k + 1] : 1 - il[k + 1] - il[nv]) * (isr ? sk : sk * ss[nv]);
+      // times s_k (s_k s_{i-1}), their exponents taken into the window's
+      double v = fix96_value(hi, lo, isr ? ew : 1) * scale_pow2(ss[k + 1], -il[k + 1]);
+      if (!isr) v *= scale_pow2(ss[nv], -il[nv]);
       if (bad) v = __longlong_as_double(0x7ff8000000000000ll);
       if (isr) {
         rv[k] = v;
-        rf[k] = (float)scale_pow2(v, -ew);  // |r_k| <= ||w|| < 2^ew
+        rf[k] = (float)scale_pow2(v, -ew);  // |r_k| <= ||w||
       } else {
         lv[k] = v;
         Lf[(size_t)(nv - 1) * (nv - 2) / 2 + k] = (float)v;
         if (b == 0) Lg[(size_t)(nv - 1) * nl + k] = v;
-        if (!(fabs(v) <= 1e-8)) s_slow = 1;
+        if (!(fabs(v) <= 1e-8) && (!bad || measure)) s_slow = 1;  // (a step that will be run again says nothing)
       }
     }
     __syncthreads();
@@ -308,7 +385,7 @@ __global__ void __launch_bounds__(kCwyThreads, 1) k_ar_cwy(KState st, CsrDev A, 
       rv[t] = h * ss[t + 1];  // c_k
     }
     if (b == 0)  // the next step's sums start at zero (no block reads or adds to them before this step's end)
-      for (int l = t; l < aw; l += bd) acc_all[(size_t)((i + 1) % 3) * aw + l] = 0;
+      for (int l = t; l < aw; l += bd) acc_all[(size_t)((rr + 1) % 3) * aw + l] = 0;
     __syncthreads();
     // ---- w -= sum_k c_k W_k, the squared norm, W_i to global memory
     {
@@ -335,46 +412,31 @@ __global__ void __launch_bounds__(kCwyThreads, 1) k_ar_cwy(KState st, CsrDev A, 
         }
         p = fma(w, w, p);
       }
-      long long w3[3];
-      const bool ok = fix144_limbs(p, 2 * ew, w3);
-      if (!ok) s_bad = 1;
+      long long w4[4];
+      if (!fix192_limbs(p, 2 * ew + 8, w4)) s_bad = 1;
 #pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        const long long v = warp_sum_s64(w3[q]);
-        if (lane == 0) red3[warp * 3 + q] = v;
+      for (int q = 0; q < 4; ++q) {  // 24 bits at a time: 32 lanes of them fit an int
+        const unsigned l = __reduce_add_sync(0xffffffffu, (unsigned)w4[q] & 0xffffffu);
+        const unsigned h = __reduce_add_sync(0xffffffffu, (unsigned)(w4[q] >> 24));
+        if (lane == 0) red4[warp * 4 + q] = (long long)l + ((long long)h << 24);
       }
       __syncthreads();
-      if (t == 0) {
-        long long q0 = 0, q1 = 0, q2 = 0;
-        for (int g = 0; g < (bd >> 5); ++g) {
-          q0 += red3[3 * g];
-          q1 += red3[3 * g + 1];
-          q2 += red3[3 * g + 2];
-        }
-        fix96_carry(q1, q0);
-        fix96_carry(q2, q1);
-        red_add_s64(acc + 4 * nl, q0);
-        red_add_s64(acc + 4 * nl + 1, q1);
-        red_add_s64(acc + 4 * nl + 2, q2);
-        if (s_bad) red_add_s64(acc + 4 * nl + 3, 1);
-        s_bad = 0;
+      if (t < 4) {  // a limb each, its carry into the next one's word
+        long long q = 0, h = 0;
+#pragma unroll 4
+        for (int g = 0; g < (bd >> 5); ++g) q += red4[4 * g + t];
+        if (t < 3) fix96_carry(h, q);
+        red_add_s64(acc + 4 * nl + t, q);
+        if (t < 3) red_add_s64(acc + 4 * nl + t + 1, h);
+        if (t == 3 && s_bad) red_add_s64(acc + 4 * nl + kCwyBadNorm, 1);
+        if (t == 3) s_bad = 0;
       }
     }
     if (!grid_sync_to(&c->bar_count, (++nb) * (unsigned)G, &c->err)) break;
-    if (i == nl && b == 0 && lead) {  // the last step's norm
-      const long long* pn = acc + 4 * nl;
-      const double beta = ld_relaxed_s64(pn + 3) != 0
-                              ? __longlong_as_double(0x7ff8000000000000ll)
-                              : sqrt(fix144_value(ld_relaxed_s64(pn + 2), ld_relaxed_s64(pn + 1), ld_relaxed_s64(pn),
-                                                  2 * ew));
-      HAT(st, i, i - 1) = beta;
-      st.s[i] = 1.0 / beta;
-      c->itx = i - 1;
-      if (beta == 0.0) c->breakdown = 1;
-      if (st.host_flag) st.host_flag[1] = i;
-      st_release_gpu(&c->pub, i - 1);
-      last = i - 1;
-    }
+    ++rr;
+    pending = true;
+    measured = measure;
+    measure = false;
   }
   if (b == 0 && lead) st_release_gpu(&c->steps_end, last + 1);
 }

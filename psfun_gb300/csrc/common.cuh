@@ -372,14 +372,14 @@ PSF_DEVINL void bulk_g2s_hint(void* dst_smem, const void* src_gmem, unsigned byt
 
 PSF_DEVINL void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// v * 2^k, exact.  For a normal v whose scaled value stays normal the scaling
+// v * 2^k.  For a normal v whose scaled value stays normal the scaling
 // is an integer add on the exponent field (INT pipe, no FP64 instruction);
 // zeros are returned as they are; subnormals, Inf/NaN and out-of-range results
-// take an exact multiply in a separate, non-inlined function, so that the
+// take ldexp (one rounding) in a separate, non-inlined function, so that the
 // compiler cannot evaluate it speculatively on the fast path (ldexp costs
 // several FP64 instructions, and the FP64 pipe is a bottleneck of the kernels
 // that scale every element).
-static __device__ __noinline__ double scale_pow2_slow(double v, int k) { return v * ldexp(1.0, k); }
+static __device__ __noinline__ double scale_pow2_slow(double v, int k) { return ldexp(v, k); }
 
 PSF_DEVINL double scale_pow2(double v, int k) {
   const long long b = __double_as_longlong(v);

@@ -66,41 +66,6 @@ PSF_DEVINL double fix96_value(long long hi, long long lo, int E) {
   return scale_pow2(fma((double)hi, 281474976710656.0, (double)lo), E - 96);
 }
 
-// A wider window for sums that may be far below their bound (the squared norm
-// of what Gram-Schmidt leaves): p 2^(144-E) as three 48-bit limbs, lowest
-// first, exact for p >= 2^(E-91); p >= 0.
-PSF_DEVINL bool fix144_limbs(double p, int E, long long (&w)[3]) {
-  const unsigned hi = (unsigned)__double2hiint(p), lo = (unsigned)__double2loint(p);
-  const int ex = (int)((hi >> 20) & 0x7ffu);
-  int pos = max(ex, 1) - (E + 931);
-  unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | (ex ? 0x100000u : 0u)) << 32) | lo;
-  const bool ok = pos <= 91 && ex != 0x7ff && (hi >> 31) == 0u;
-  const bool top = pos >= 48;
-  if (top) pos -= 48;
-  m >>= min(max(-pos, 0), 63);
-  const int ls = min(max(pos, 0), 47);
-  const long long l = (long long)((m << ls) & (unsigned long long)kFixMask48), h = (long long)(m >> (48 - ls));
-  w[0] = top ? 0 : l;
-  w[1] = top ? l : h;
-  w[2] = top ? h : 0;
-  return ok;
-}
-
-PSF_DEVINL double fix144_value(long long w2, long long w1, long long w0, int E) {
-  w1 += w0 >> 48;
-  w0 &= kFixMask48;
-  w2 += w1 >> 48;
-  w1 &= kFixMask48;
-  const double c = 281474976710656.0;  // 2^48
-  return scale_pow2(fma(fma((double)w2, c, (double)w1), c, (double)w0), E - 144);
-}
-
-PSF_DEVINL long long warp_sum_s64(long long v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
 PSF_DEVINL void red_add_s64(long long* p, long long v) {
   asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
@@ -130,6 +95,17 @@ PSF_DEVINL bool fix192_limbs(double p, int E, long long (&w)[4]) {
   w[2] = q == 1 ? h : q == 2 ? l : 0;
   w[3] = q == 2 ? h : 0;
   return ok;
+}
+
+// The value of N 48-bit limbs, lowest first, in units of their window.
+template <int N>
+PSF_DEVINL double fix_units(long long (&w)[N]) {
+#pragma unroll
+  for (int q = 0; q + 1 < N; ++q) fix96_carry(w[q + 1], w[q]);
+  double v = (double)w[N - 1];
+#pragma unroll
+  for (int q = N - 2; q >= 0; --q) v = fma(v, 281474976710656.0, (double)w[q]);  // 2^48
+  return v;
 }
 
 // A non-zero addend with a mantissa bit below a window's unit 2^U.
@@ -215,14 +191,7 @@ PSF_DEVINL bool count_wait(const long long* words, int G, double& units, bool& s
 #pragma unroll
   for (int q = 0; q + 1 < N; ++q) w[q] = (w[q] & (kCountOne - 1)) - kCountLowBias;
   w[N - 1] = (w[N - 1] & (kCountCut - 1)) - kCountTopBias;
-#pragma unroll
-  for (int q = 0; q + 1 < N; ++q) {
-    w[q + 1] += w[q] >> 48;
-    w[q] &= kFixMask48;
-  }
-  units = (double)w[N - 1];
-#pragma unroll
-  for (int q = N - 2; q >= 0; --q) units = fma(units, 281474976710656.0, (double)w[q]);  // 2^48
+  units = fix_units(w);
   stands = flags == 0u;
   if (!stands) stands = flags < 0x100u && fabs(units) >= 4611686018427387904.0;  // no bad addend, 2^62
   return true;

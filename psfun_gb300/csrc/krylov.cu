@@ -1491,11 +1491,11 @@ static int lz_norm_exponent(double norm_inf) {
   return norm_inf > 0.0 ? (std::isfinite(norm_inf) ? std::ilogb(norm_inf) + 1 : 1000) : 0;
 }
 
-// ||w|| <= |scaling| ||A||_2 ||v||, ||A||_2 <= sqrt(n) ||A||_inf; 2^ew bounds it
-// with a bit to spare.
-static int cwy_norm_exponent(double scaling, double norm_inf, int64_t n) {
-  const double bound = std::fabs(scaling) * norm_inf * std::sqrt((double)n);
-  return bound > 0.0 ? (std::isfinite(bound) ? std::ilogb(bound) + 2 : 1000) : 0;
+// The first window of k_ar_cwy: ||w|| <= |scaling| ||A||_2 ||v||, as large as
+// ||A||_inf where A is not far from symmetric, and a bit to spare.
+static int cwy_norm_exponent(double scaling, double norm_inf) {
+  const double bound = std::fabs(scaling) * norm_inf;
+  return bound > 0.0 ? (std::isfinite(bound) ? std::max(std::ilogb(bound) + 2, kCwyMinExp) : 1000) : 0;
 }
 
 // Steps [i_begin, i_end) in one cooperative launch; with a monitor the grid
@@ -1827,7 +1827,7 @@ int krylov_apply_device(psfun_krylov* meth, psfun_serial* fun, psfun_csr* a, dou
     mon.scr_stride = lz_scr_stride;
     mon.count = kCwyMonitors;
     double sc = scaling;
-    int ew = cwy_norm_exponent(scaling, a->norm_inf, n);
+    int ew = cwy_norm_exponent(scaling, a->norm_inf);
     int monitors = istop == 1 ? kCwyMonitors : 0;
     int chunk = cwy.chunk, rt = cwy.rt;
     long long* acc = reinterpret_cast<long long*>(st.coef + (ldh + 2));
@@ -1865,7 +1865,7 @@ int krylov_apply_device(psfun_krylov* meth, psfun_serial* fun, psfun_csr* a, dou
     key.order = A.order; key.sched = A.sched; key.nnz = A.nnz; key.ntiles = A.ntiles; key.stream = A.stream;
     // the windows of the sums follow the norm of the matrix
     key.max_row = a->max_row; key.ea = lz_norm_exponent(a->norm_inf);
-    key.ew = cwy_norm_exponent(scaling, a->norm_inf, n);
+    key.ew = cwy_norm_exponent(scaling, a->norm_inf);
     key.a = a; key.x = x; key.y = y; key.arnoldi = arnoldi;
     key.keeplast = meth->keeplast; key.gs = gs; key.gv = gv; key.gm = gm; key.fp = fpk; key.scaling = scaling;
     key.cwy.G = cwy.G; key.cwy.chunk = cwy.chunk; key.cwy.rt = cwy.rt; key.cwy.threads = cwy.threads;
