@@ -51,3 +51,19 @@ def test_scales_whose_product_overflows(lib, orc, xs, As):
     """1 / (||W_j|| ||W_k||) is beyond the largest double."""
     A = As * matrices.laplacian_2d(40)
     check(orc, sp.csr_matrix(A), xs * np.random.default_rng(2).standard_normal(1600), "ARNOLDI", "GENPADE", 2, m=12)
+
+
+@pytest.mark.parametrize("delta", [1e-3, 1e-4, 1e-5, 1e-6, 1e-7])
+def test_orthogonality_lost_by_degrees(lib, delta):
+    """x is an eigenvector up to delta: the second basis vector has lost
+    eps / delta of its orthogonality, on either side of where the coefficients'
+    correction leaves FP32.  The result is exp(A) x all the same."""
+    d = -np.linspace(0.0, 4.0, 4001)
+    x = delta * np.random.default_rng(3).standard_normal(d.size)
+    x[-1] = 1.0
+    import psfun_gb300 as pg
+    fun = pg.PsfunDSerial()
+    assert fun.set("VARIANT", "GENPADE") == 0
+    r = pg.PsfunDKrylov().apply(fun, pg.CsrMatrix.from_scipy(sp.diags(d).tocsr()), x, 1e-12, itmax=30, istop=2)
+    y = np.exp(d) * x
+    assert r.info == 0 and np.linalg.norm(r.y - y) <= 1e-10 * np.linalg.norm(y)
