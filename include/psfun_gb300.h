@@ -87,8 +87,8 @@ int psfun_gpu_profile_enable(int on);
 int psfun_gpu_profile_read(int kernel, long long* launches, double* total_ms);
 /* No counterpart in the reference.  Runs a device wait that nothing completes
  * (which 0: a grid barrier short of one arrival; 1: an mbarrier phase nobody
- * completes) through the same bounded-wait code as the solvers, so that a
- * test can see the limit expire: returns PSFUN_ERR_DEVICE_TIMEOUT after about
+ * completes; 2: a batch monitor whose step nobody publishes) through the same
+ * bounded-wait code as the solvers, so that a test can see the limit expire: returns PSFUN_ERR_DEVICE_TIMEOUT after about
  * two seconds, with the CUDA context still usable. */
 int psfun_gpu_selftest_wait(int which);
 

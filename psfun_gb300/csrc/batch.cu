@@ -823,24 +823,30 @@ PSF_DEVINL void batch_monitor(const BatchArgs& B, int mb) {
   for (long long task = w; task < total; task += nw) {
     const int i = 1 + (int)(task / B.count);
     const BInst& I = B.inst[task % B.count];
-    unsigned p = ld_acquire_gpu(&I.cnt[2]);
-    if ((p & ~kPubEnd) < (unsigned)i && !(p & kPubEnd)) {
+    // lane 0 waits and decides for the warp: the word and the error flag change
+    // meanwhile, and lanes that left on their own would be missing from the
+    // others' warp-wide operations
+    int pub = -1;  // -1: the wait gave up, or another one did
+    if ((threadIdx.x & 31) == 0) {
+      unsigned p = ld_acquire_gpu(&I.cnt[2]);
+      bool ok = true;
       const unsigned long long t0 = globaltimer_ns();
-      do {
+      while (ok && (p & ~kPubEnd) < (unsigned)i && !(p & kPubEnd)) {
         __nanosleep(200);
-        if (*(volatile int*)B.err != 0) return;
-        if (globaltimer_ns() - t0 > kWaitLimitNs) {
+        if (*(volatile int*)B.err != 0) {
+          ok = false;
+        } else if (globaltimer_ns() - t0 > kWaitLimitNs) {
           atomicOr(B.err, DEVERR_TIMEOUT);
-          return;
+          ok = false;
         }
         p = ld_acquire_gpu(&I.cnt[2]);
-      } while ((p & ~kPubEnd) < (unsigned)i && !(p & kPubEnd));
+      }
+      if (ok) pub = (int)(p & ~kPubEnd);
     }
-    __threadfence();
     __syncwarp();
-    // (lanes may have read different values: the decision is the lowest)
-    const unsigned pub = __reduce_min_sync(0xffffffffu, p & ~kPubEnd);
-    if (pub >= (unsigned)i) warp_estimate<R>(I, i, B, scr);
+    pub = __shfl_sync(0xffffffffu, pub, 0);
+    if (pub < 0) return;
+    if (pub >= i) warp_estimate<R>(I, i, B, scr);
   }
 }
 
@@ -1254,9 +1260,27 @@ static int batch_launch(BatchArgs& B, std::vector<BInst>& hinst, BInst* dinst, c
   return PSFUN_SUCCESS;
 }
 
-}  // namespace psf
+// One monitor block that waits for a step which nobody publishes (the failure
+// test of psfun_gpu_selftest_wait).
+__global__ void __launch_bounds__(kBatchThreads, 1) k_selftest_monitor(BatchArgs B) { batch_monitor<1>(B, 0); }
 
-namespace psf {
+int batch_selftest_monitor(double* buf, int** err, cudaStream_t s) {
+  BInst I;
+  memset(&I, 0, sizeof I);
+  BatchArgs B;
+  memset(&B, 0, sizeof B);
+  B.inst = reinterpret_cast<BInst*>(buf + 16);
+  B.err = reinterpret_cast<int*>(buf);
+  I.cnt = reinterpret_cast<unsigned*>(buf + 8);
+  B.count = 1;
+  B.nl = 4;
+  B.monitors = 1;
+  PSF_CUDA(cudaMemcpyAsync(B.inst, &I, sizeof I, cudaMemcpyHostToDevice, s));
+  k_selftest_monitor<<<1, kBatchThreads, 0, s>>>(B);
+  PSF_CUDA(cudaGetLastError());
+  *err = B.err;
+  return PSFUN_SUCCESS;
+}
 
 // One batch item, from either entry point: f(tA)X (N = 0) or the quadrature
 // sum over N shifts.

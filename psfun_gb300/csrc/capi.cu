@@ -160,8 +160,8 @@ bool parse_fun(const psfun_serial* fun, FunParams* fp) {
 // Self-test of the bounded device waits: a wait that nothing completes.
 // which 0: a grid barrier of a 2-CTA cooperative grid whose target is one
 // arrival more than the grid makes; which 1: an mbarrier wait for a phase
-// that no thread or copy completes.  Both give up after kWaitLimitNs and
-// record DEVERR_TIMEOUT, as every wait of the solvers does.
+// that no thread or copy completes (2: k_selftest_monitor of batch.cu).  They
+// give up after kWaitLimitNs and record DEVERR_TIMEOUT, as every wait of the solvers does.
 __global__ void k_selftest_wait(int which, unsigned* counter, int* err) {
   __shared__ uint64_t bar;
   if (which == 0) {
@@ -184,18 +184,20 @@ using namespace psf;
 extern "C" {
 
 int psfun_gpu_selftest_wait(int which) {
-  if (which < 0 || which > 1) return PSFUN_ERR_INVALID_ARGS_COMBINATION;
+  if (which < 0 || which > 2) return PSFUN_ERR_INVALID_ARGS_COMBINATION;
   static DevBuf buf;
-  PSF_TRY(buf.ensure(64));
+  PSF_TRY(buf.ensure(4096));
   cudaStream_t s = stream();
-  PSF_CUDA(cudaMemsetAsync(buf.ptr, 0, 64, s));
+  PSF_CUDA(cudaMemsetAsync(buf.ptr, 0, 4096, s));
   unsigned* counter = buf.as<unsigned>();
   int* err = reinterpret_cast<int*>(counter + 4);
   if (which == 0) {
     void* args[] = {(void*)&which, (void*)&counter, (void*)&err};
     PSF_CUDA(cudaLaunchCooperativeKernel((void*)k_selftest_wait, dim3(2), dim3(32), args, 0, s));
-  } else {
+  } else if (which == 1) {
     k_selftest_wait<<<1, 32, 0, s>>>(which, counter, err);
+  } else {
+    PSF_TRY(batch_selftest_monitor(buf.as<double>(), &err, s));
   }
   count_launch();
   PSF_CUDA(cudaGetLastError());
