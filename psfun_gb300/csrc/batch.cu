@@ -95,7 +95,13 @@ struct BatchArgs {
   const int* tile_inst;  // instance of every global tile
   int chunk;             // tiles per queue grab (1..kBatchChunkMax)
   int monitors;          // blocks of the grid that run the estimates (its last ones)
-  zc* mon_scr;           // per monitor warp: 7 R pole scratches, then R yk (batch_mon_zc)
+  zc* mon_scr;           // per warp that estimates: 7 R pole scratches, then R yk (batch_mon_zc)
+  // Estimates are numbered with the instances fastest; *ticket is the first
+  // that nobody has taken, help[0..1] and help[2..3] in turn the range that the
+  // step blocks take, help[4] 1 + the last step once the steps have ended
+  int helpers;           // their warps that estimate (0: none)
+  int lag;               // estimates that may wait for the monitors
+  unsigned long long *ticket, *help;
 };
 
 constexpr unsigned kPubEnd = 0x80000000u;
@@ -751,9 +757,10 @@ PSF_DEVINL void finalize(const BInst& I, int ph, int i, const BatchArgs& B, doub
 // of an instance, by one warp: the 7 R pole solves on a lane each, then
 // lane q the sums of pair q.
 template <int R>
-PSF_DEVINL void warp_estimate(const BInst& I, int i, const BatchArgs& B, zc* scr) {
+static __device__ __noinline__ void warp_estimate(const BInst* inst, int i, int nl, double eps, zc* scr) {
   static_assert(7 * R <= 32, "one pole per lane");
-  const int nl = B.nl, lane = threadIdx.x & 31;
+  const BInst& I = *inst;
+  const int lane = threadIdx.x & 31;
   const size_t stride = (size_t)(nl + 2);
   double* yk = reinterpret_cast<double*>(scr + (size_t)R * 7 * 5 * stride);  // R rows of 2 ((nl + 3) / 2)
   const size_t ldy = 2 * (size_t)((nl + 3) / 2);
@@ -797,30 +804,32 @@ PSF_DEVINL void warp_estimate(const BInst& I, int i, const BatchArgs& B, zc* scr
     e[1] = errden;
     const double ratio = errnum / errden;
     pa(I, q, PA_RS, nl)[i + 1] = ratio;
-    if (ratio < B.eps) atomicMin(&I.conv[q], 2 * i);
+    if (ratio < eps) atomicMin(&I.conv[q], 2 * i);
   }
   __syncwarp();
 }
 
-// A monitor block: estimates (instance k, step i), counted with the instances
-// fastest, go to the monitor warps of the grid in turn; each waits (bounded)
-// until its step is published, or leaves it out when the instance has ended
-// before.  The steps do not wait for the estimates: a pair whose estimate
-// converges meanwhile stops a step or two later, which changes nothing that
-// its result uses (later basis slots and entries of T), and the first
-// converged iteration is the one taken, as in the serial order.  On the
-// finalising block an estimate of order 18 costs ~40 us between two grid
-// barriers, with every other SM waiting; 24 uneven graphs (2-65 thousand
-// rows, 4 right-hand sides): 7.60 -> 4.87 ms with the cheaper
-// phases below, 7.0 by the monitors alone.
+// A monitor block: its warps take the estimates (instance k, step i), counted
+// with the instances fastest, in turn; each waits (bounded) until its step is
+// published, or leaves it out when the instance has ended before.  The steps
+// do not wait for the estimates: a pair whose estimate converges meanwhile
+// stops a step or two later, which changes nothing that its result uses (later
+// basis slots and entries of T), and the first converged iteration is the one
+// taken, as in the serial order.  On the finalising block an estimate of order
+// 18 costs ~40 us between two grid barriers, with every other SM waiting; 24
+// uneven graphs (2-65 thousand rows, 4 right-hand sides), the mapping with a
+// thread per row: 7.6 -> 4.9 ms with the cheaper phases below.
 template <int R>
 PSF_DEVINL void batch_monitor(const BatchArgs& B, int mb) {
   const int warp = threadIdx.x >> 5;
   if (warp >= kBatchMonWarps) return;
-  const int w = mb * kBatchMonWarps + warp, nw = B.monitors * kBatchMonWarps;
-  zc* scr = B.mon_scr + (size_t)w * batch_mon_zc(R, B.nl);
+  zc* scr = B.mon_scr + (size_t)(mb * kBatchMonWarps + warp) * batch_mon_zc(R, B.nl);
   const long long total = (long long)B.count * (B.nl - 1);
-  for (long long task = w; task < total; task += nw) {
+  for (;;) {
+    long long task = 0;
+    if ((threadIdx.x & 31) == 0) task = (long long)atomicAdd(B.ticket, 1ull);
+    task = __shfl_sync(0xffffffffu, task, 0);
+    if (task >= total) return;
     const int i = 1 + (int)(task / B.count);
     const BInst& I = B.inst[task % B.count];
     // lane 0 waits and decides for the warp: the word and the error flag change
@@ -846,7 +855,46 @@ PSF_DEVINL void batch_monitor(const BatchArgs& B, int mb) {
     __syncwarp();
     pub = __shfl_sync(0xffffffffu, pub, 0);
     if (pub < 0) return;
-    if (pub >= i) warp_estimate<R>(I, i, B, scr);
+    if (pub >= i) {
+      warp_estimate<R>(&I, i, B.nl, B.eps, scr);
+    } else {  // no estimate of this step; of none once all steps have ended before
+      const unsigned long long e = *(volatile unsigned long long*)&B.help[4];
+      if (__any_sync(0xffffffffu, e != 0 && (unsigned long long)i >= e)) return;
+    }
+  }
+}
+
+// The monitors' 60 warps do ~1.5 estimates per us at order 18, fewer at higher
+// orders; many small instances publish more.  After step i block 0 looks how
+// many estimates of published steps (all up to i - 1; i at the end) nobody has
+// taken.  When they are B.lag it takes them off the ticket, and after the
+// barrier every block does its share, on one warp per sub-partition: a step is
+// then held for a few estimates' time, and the blocks that wait for the
+// monitors at the end wait for a few each.  128 instances of 400 rows, 200
+// steps that do not converge: 25.4 ms, 95.7 by the monitors alone, 52.5 with
+// every estimate on its finalising block.
+PSF_DEVINL void batch_hand_over(const BatchArgs& B, int upto, int slot, bool end) {
+  const unsigned long long lim = (unsigned long long)upto * B.count;
+  const unsigned long long t = *(volatile unsigned long long*)B.ticket;
+  unsigned long long from = lim;
+  if (t < lim && lim - t >= (unsigned long long)B.lag) from = atomicMax(B.ticket, lim);
+  volatile unsigned long long* h = B.help + 2 * slot;
+  h[0] = from;
+  h[1] = lim;
+  if (end) *(volatile unsigned long long*)&B.help[4] = (unsigned long long)upto + 1;
+}
+
+template <int R>
+PSF_DEVINL void batch_help(const BatchArgs& B, int slot, int G) {
+  const int w = (int)(threadIdx.x >> 5) * G + (int)blockIdx.x;  // the blocks first
+  if ((int)(threadIdx.x >> 5) >= kBatchMonWarps || w >= B.helpers) return;
+  const volatile unsigned long long* h = B.help + 2 * slot;
+  const unsigned long long from = h[0], to = h[1];
+  zc* scr = B.mon_scr + (size_t)(B.monitors * kBatchMonWarps + w) * batch_mon_zc(R, B.nl);
+  for (unsigned long long task = from + w; task < to; task += B.helpers) {
+    const int i = 1 + (int)(task / B.count);
+    const BInst* I = &B.inst[task % B.count];
+    if ((int)(*(volatile unsigned*)&I->cnt[2] & ~kPubEnd) >= i) warp_estimate<R>(I, i, B.nl, B.eps, scr);
   }
 }
 
@@ -1123,7 +1171,7 @@ __global__ void __launch_bounds__(kBatchThreads, 1) k_batch(BatchArgs B) {
   if (blockIdx.x >= G) {
     batch_monitor<R>(B, blockIdx.x - G);
   } else {
-    int ph_idx = 0;
+    int ph_idx = 0, ran = 0;
     run_phase<R>(B, PH_INIT, 0, &B.queue[ph_idx++], sm);
     if (!gsync()) return;
     __shared__ unsigned act;
@@ -1134,7 +1182,15 @@ __global__ void __launch_bounds__(kBatchThreads, 1) k_batch(BatchArgs B) {
       run_phase<R>(B, PH_SPMM, i, &B.queue[ph_idx++], sm);
       if (!gsync()) return;
       run_phase<R>(B, PH_UPDATE, i, &B.queue[ph_idx++], sm);
+      if (B.helpers > 0 && blockIdx.x == 0 && threadIdx.x == 0) batch_hand_over(B, i - 1, i & 1, false);
       if (!gsync()) return;
+      if (B.helpers > 0) batch_help<R>(B, i & 1, G);
+      ran = i;
+    }
+    if (B.helpers > 0) {
+      if (blockIdx.x == 0 && threadIdx.x == 0) batch_hand_over(B, ran, (ran + 1) & 1, true);
+      if (!gsync()) return;
+      batch_help<R>(B, (ran + 1) & 1, G);
     }
   }
   // the steps and every estimate are done: final f per instance (CTA k
@@ -1250,6 +1306,7 @@ static int batch_launch(BatchArgs& B, std::vector<BInst>& hinst, BInst* dinst, c
   if (per < 1) per = 1;
   int G = std::max(1, sm_count() * per - B.monitors);
   if (G > B.total_tiles) G = std::max(1, B.total_tiles);
+  B.helpers = std::min(B.helpers, kBatchMonWarps * G);
   // about four grabs per block and phase, at most kBatchChunkMax tiles each:
   // larger grabs amortise the queue and per-run costs, smaller ones balance
   B.chunk = std::max(1, std::min(kBatchChunkMax, B.total_tiles / (4 * G)));
@@ -1275,6 +1332,8 @@ int batch_selftest_monitor(double* buf, int** err, cudaStream_t s) {
   B.count = 1;
   B.nl = 4;
   B.monitors = 1;
+  B.ticket = reinterpret_cast<unsigned long long*>(buf + 2);
+  B.help = B.ticket + 1;
   PSF_CUDA(cudaMemcpyAsync(B.inst, &I, sizeof I, cudaMemcpyHostToDevice, s));
   k_selftest_monitor<<<1, kBatchThreads, 0, s>>>(B);
   PSF_CUDA(cudaGetLastError());
@@ -1339,7 +1398,16 @@ static int batch_run(DevBuf* wsbuf, int keeplast, int mapping, int count, const 
   const bool estimates = istop == 1 && items[0].N == 0;
   const int monitors =
       estimates ? std::max(1, std::min(sm_count() / 10, (3 * count + kBatchMonWarps - 1) / kBatchMonWarps)) : 0;
-  const size_t oMon = carve((size_t)monitors * kBatchMonWarps * batch_mon_zc(R, nl) * 2);
+  // Warps of the step blocks that estimate when the monitors lag: as many as
+  // there may be, within 1 GB of scratch.  They are called in when the lag is
+  // one estimate for each of them and eight for each monitor's warp (a short
+  // solve of few instances never gets there), and not needed where all
+  // estimates together are not more.
+  const int64_t hmax = std::min<int64_t>((int64_t)kBatchMonWarps * std::min(sm_count(), std::max(tiles, 1)),
+                                         std::max<int64_t>(1, ((int64_t)1 << 30) / (int64_t)(batch_mon_zc(R, nl) * sizeof(zc))));
+  const int64_t lag = std::max<int64_t>(hmax, (int64_t)8 * kBatchMonWarps * monitors);
+  const int helpers = estimates && (int64_t)count * (nl - 1) > lag ? (int)hmax : 0;
+  const size_t oMon = carve(((size_t)monitors * kBatchMonWarps + helpers) * batch_mon_zc(R, nl) * 2);
   const size_t oConv = carve(((size_t)count * R + 1) / 2);
   const size_t oInst = carve((sizeof(BInst) * count + 7) / 8);
   const size_t oQ = carve(2 * (size_t)nl + 8);
@@ -1400,6 +1468,10 @@ static int batch_run(DevBuf* wsbuf, int keeplast, int mapping, int count, const 
   B.active = misc + 3;
   B.tile_inst = dti;
   B.monitors = monitors;
+  B.helpers = helpers;
+  B.lag = (int)lag;
+  B.ticket = reinterpret_cast<unsigned long long*>(misc + 4);
+  B.help = B.ticket + 1;
   B.mon_scr = reinterpret_cast<zc*>(base + oMon);
   const unsigned active = (unsigned)count;
   PSF_CUDA(cudaMemcpyAsync(B.active, &active, sizeof active, cudaMemcpyHostToDevice, s));
