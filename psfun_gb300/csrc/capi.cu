@@ -606,7 +606,7 @@ int spmv_device(psfun_csr* a, double alpha, const double* x, double beta, double
     const int tpc = std::max(1, (a->ntiles + gmax - 1) / gmax);
     const int g = std::max(1, (a->ntiles + tpc - 1) / tpc);
     if (a->order)
-      k_spmv_axpby<true><<<g, kSpmvThreads, kLzSmemBytes, s>>>(a->dev(), x, alpha, beta, y, errbuf.as<int>(), tpc);
+      k_spmv_axpby<true><<<g, kSpmvThreads, kLzSmemBytes, s>>>(a->dev(true), x, alpha, beta, y, errbuf.as<int>(), tpc);
     else
       k_spmv_axpby<false><<<g, kSpmvThreads, kLzSmemBytes, s>>>(a->dev(), x, alpha, beta, y, errbuf.as<int>(), tpc);
     count_launch();

@@ -126,12 +126,14 @@ struct psfun_csr {
   double* bj_udinv = nullptr;
   int sym = -1;                // A == A^T (pattern and values): 1 yes, 0 no, -1 not yet checked
   psfun_csr* T = nullptr;      // A^T as its own handle, built on first use (nonsymmetric A)
-  psf::CsrDev dev() const {
+  // with_order: for the plain product alone, which reads it; the tile copies
+  // of the other kernels take the order's 2 bytes a row along when it is there
+  psf::CsrDev dev(bool with_order = false) const {
     psf::CsrDev d;
     d.n = n; d.nnz = nnz; d.irp = irp; d.ja = ja; d.val = val; d.tile_row = tile_row; d.ntiles = ntiles;
     d.sched = sched;
     d.tile_desc = tile_desc;
-    d.order = order;
+    d.order = with_order ? order : nullptr;
     d.stream = (nnz * 12 + n * 4) > ((int64_t)64 << 20) ? 1 : 0;
     return d;
   }
