@@ -246,8 +246,9 @@ int psfun_gpu_profile_read(int kernel, long long* launches, double* total_ms) {
 }  // extern "C"
 
 // ---- CSR ------------------------------------------------------------------
-// f(begin, end) over [0, n) in contiguous parts on up to 16 host threads
-// (one part below 2^17 items).
+// f(begin, end) over [0, n) in contiguous parts on up to 16 host threads (one
+// part below 2^17 items).  Parts begin at multiples of 32, so that what f counts
+// over 32 items at a time does not depend on the number of threads.
 template <class F>
 static void host_parallel_for(int64_t n, F f) {
   const int T = std::max(1, std::min(16, (int)std::thread::hardware_concurrency()));
@@ -257,7 +258,7 @@ static void host_parallel_for(int64_t n, F f) {
   }
   std::vector<std::thread> th;
   th.reserve(T);
-  for (int t = 0; t < T; ++t) th.emplace_back([&, t] { f(n * t / T, n * (t + 1) / T); });
+  for (int t = 0; t < T; ++t) th.emplace_back([&, t] { f(n * t / T & ~(int64_t)31, t + 1 < T ? n * (t + 1) / T & ~(int64_t)31 : n); });
   for (auto& x : th) x.join();
 }
 
