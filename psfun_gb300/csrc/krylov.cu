@@ -68,6 +68,7 @@ constexpr int kMgsThreads = 1024;
 // alpha (0), CTA 0's answer to a stop request (2) and the four limbs of the
 // norm (4) on a 64-byte line, then the arrivals of the FP64 sums of alpha (8)
 // and of the norm (9).
+constexpr int kLzNext = 4;  // bits that alpha and beta may grow by in a step
 constexpr int kLzWordsAt = 4096, kLzBuf = 16, kLzUsed = 10, kLzWords = 3 * kLzBuf;
 __host__ __device__ constexpr long long lz_word_start(int q) {
   return q < 2 ? count_start(q, 2) : q >= 4 && q < 8 ? count_start(q - 4, 4) : 0;
@@ -134,14 +135,15 @@ __global__ void __launch_bounds__(kVecThreads) k_init(KState st, const double* _
 //            reads W_{i+1} of other CTAs
 // (fixed-point sums that count their arrivals, fixsum.cuh).  Every CTA derives
 // the scalars itself, so none is re-read from memory, and CTA 0 records H, s
-// and itx for the estimate / final kernels.  The windows of the sums come from
-// ||A||_2 <= ||A||_inf < 2^ea for a symmetric A: |W.u| <= 2^ea ||W||^2, and
-// ||w|| <= 5 2^ea ||W|| as c2 W_{i-1} is the previous step's ||w|| long;
-// ||W|| = 1 / s_i.  A unit of alpha is then 2^(ea-78), one of beta^2
-// 2^(2 ea-168) (unit vectors).  Sums far below the bound that have lost bits
-// (alpha below 2^(ea-16), beta below 2^(ea-53): vectors that do not meet the
-// rows of the norm), or above it (A not symmetric), are taken again in FP64
-// from the CTAs' partials (count_sum_fp64), by all CTAs alike.  Measured:
+// and itx for the estimate / final kernels.  The windows of the sums: with 2^ew
+// a bound of the step's alpha and beta (unit vectors, ||W|| = 1 / s_i), a unit
+// of alpha is 2^(ew-78), one of beta^2 2^(2 ew-168).  The first step takes
+// ||A||_inf for the bound, each other one 2^kLzNext times what the step before
+// gave: ||A|| may be far above it, where the vectors do not meet the rows of
+// the norm.  A sum that has lost bits (alpha below 2^(ew-16), beta below
+// 2^(ew-53)) or lies above its window (A not symmetric, a jump of the scale) is
+// taken again in FP64 from the CTAs' partials (count_sum_fp64), by all CTAs
+// alike, for ~3 us.  Measured:
 // 100 x 100, istop 1: 0.321 -> 0.298 ms; multi-shift on 96^3, 438 steps: 15.03 ->
 // 14.61.
 // ---------------------------------------------------------------------------
@@ -276,6 +278,7 @@ PSF_DEVINL void lz_persist_body(KState& st, const CsrDev& A, int i_begin, int i_
   double sc = st.s[i_begin];  // s_i (formed by the scalar thread; others read it after each reduction)
   int k2 = 0;                 // floor(log2 s) of the previous step
   long long* const words = reinterpret_cast<long long*>(st.partials + kLzWordsAt);
+  if (threadIdx.x == kConsumerWarps * 32 + 1) sm.window = ea;  // this thread's to write
   double sprev = (i_begin >= 2) ? st.s[i_begin - 1] : 0.0;
   double beta_i = (i_begin >= 2) ? HAT(st, i_begin - 1, i_begin) : 0.0;
   double* __restrict__ u = st.u;
@@ -297,6 +300,9 @@ PSF_DEVINL void lz_persist_body(KState& st, const CsrDev& A, int i_begin, int i_
       if (i > i_begin) {
         sc = 1.0 / ldexp(sm.scal[5], k2);
         if (bid == 0) st.s[i] = sc;
+        // the window, from alpha and beta of the previous step (zeros tell nothing)
+        const unsigned m = max((unsigned)__double2hiint(sm.scal[2]) & 0x7fffffffu, (unsigned)__double2hiint(sm.scal[3]));
+        if (m > 0xfffffu) sm.window = (int)(m >> 20) - 1022 + kLzNext;
       }
       sm.scal[0] = sc;
       sm.scal[1] = (i >= 2) ? beta_i * sprev / sc : 0.0;
@@ -314,7 +320,7 @@ PSF_DEVINL void lz_persist_body(KState& st, const CsrDev& A, int i_begin, int i_
       bool up = true, stands = true;
       if (threadIdx.x == 0) {
         sc = sm.scal[0];
-        const int E = ea - 2 * ilog2_normal(sc) + 1 + kCountHeadBits;
+        const int E = sm.window - 2 * ilog2_normal(sc) + 1 + kCountHeadBits;
         long long w[2];
         {
           int b[4];
@@ -426,7 +432,7 @@ PSF_DEVINL void lz_persist_body(KState& st, const CsrDev& A, int i_begin, int i_
         }
       };
       if (threadIdx.x == 0) {
-        const int E = 2 * (ea - k2 + 3) + 1 + kCountHeadBits;
+        const int E = 2 * (sm.window - k2 + 3) + 1 + kCountHeadBits;
         long long w[4];
         fix192_limbs(S, E, w);
         double sum = 0.0;
@@ -1486,7 +1492,7 @@ static int persist_grid() {
   return g;
 }
 
-// ||A||_2 <= ||A||_inf < 2^ea for a symmetric A (see k_lz_persist).
+// The first window of k_lz_persist: ||A||_2 <= ||A||_inf < 2^ea for a symmetric A.
 static int lz_norm_exponent(double norm_inf) {
   return norm_inf > 0.0 ? (std::isfinite(norm_inf) ? std::ilogb(norm_inf) + 1 : 1000) : 0;
 }
