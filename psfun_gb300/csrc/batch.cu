@@ -1394,7 +1394,10 @@ static int batch_run(DevBuf* wsbuf, int keeplast, int mapping, int count, const 
     oE[k] = carve(items[k].N > 0 ? 0 : (size_t)R * 2 * (nl + 2));
   }
   // Monitor blocks: three warps per instance cover a step (>= 12 us) for
-  // estimates of up to ~36 us, at most a tenth of the SMs.
+  // estimates of up to ~36 us, at most a tenth of the SMs (more instances'
+  // estimates go to the step blocks, batch_hand_over).  Against estimates on the
+  // finalising blocks, four right-hand sides, 400 rows each: 8 instances 0.84 ms
+  // (1.59), 64 1.71 (2.41), 400 8.29 (10.2).
   const bool estimates = istop == 1 && items[0].N == 0;
   const int monitors =
       estimates ? std::max(1, std::min(sm_count() / 10, (3 * count + kBatchMonWarps - 1) / kBatchMonWarps)) : 0;
@@ -1403,8 +1406,8 @@ static int batch_run(DevBuf* wsbuf, int keeplast, int mapping, int count, const 
   // one estimate for each of them and eight for each monitor's warp (a short
   // solve of few instances never gets there), and not needed where all
   // estimates together are not more.
-  const int64_t hmax = std::min<int64_t>((int64_t)kBatchMonWarps * std::min(sm_count(), std::max(tiles, 1)),
-                                         std::max<int64_t>(1, ((int64_t)1 << 30) / (int64_t)(batch_mon_zc(R, nl) * sizeof(zc))));
+  const int64_t fit = std::max<int64_t>(1, ((int64_t)1 << 30) / (int64_t)(batch_mon_zc(R, nl) * sizeof(zc)));
+  const int64_t hmax = std::min<int64_t>((int64_t)kBatchMonWarps * std::min(sm_count(), std::max(tiles, 1)), fit);
   const int64_t lag = std::max<int64_t>(hmax, (int64_t)8 * kBatchMonWarps * monitors);
   const int helpers = estimates && (int64_t)count * (nl - 1) > lag ? (int)hmax : 0;
   const size_t oMon = carve(((size_t)monitors * kBatchMonWarps + helpers) * batch_mon_zc(R, nl) * 2);

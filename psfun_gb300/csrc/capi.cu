@@ -258,7 +258,8 @@ static void host_parallel_for(int64_t n, F f) {
   }
   std::vector<std::thread> th;
   th.reserve(T);
-  for (int t = 0; t < T; ++t) th.emplace_back([&, t] { f(n * t / T & ~(int64_t)31, t + 1 < T ? n * (t + 1) / T & ~(int64_t)31 : n); });
+  auto cut = [&](int t) { return t < T ? (n * t / T) & ~(int64_t)31 : n; };
+  for (int t = 0; t < T; ++t) th.emplace_back([&, t] { f(cut(t), cut(t + 1)); });
   for (auto& x : th) x.join();
 }
 

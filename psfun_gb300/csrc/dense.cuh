@@ -1508,8 +1508,8 @@ PSF_DEVINL void cta_sym_eig(int m, const double* A, int lda, double* w, double* 
 // `tridiag` tells that H is symmetric tridiagonal (Lanczos).  x and y must not
 // alias scratch.  USERF is not handled here (its f lives on the host).
 // Returns 0 or DEVERR_* flags.
-static __device__ __noinline__ int fh_apply_cta(const FunParams& fp, int m, const double* H, int ldh, const double* x, double* y,
-                            double* scratch, bool tridiag, DenseSmem& sm) {
+static __device__ __noinline__ int fh_apply_cta(const FunParams& fp, int m, const double* H, int ldh, const double* x,
+                                                double* y, double* scratch, bool tridiag, DenseSmem& sm) {
   if (m < 1) return DEVERR_BADSIZE;
   const size_t mm = (size_t)m * m;
   {  // the Pade variants' work matrices in shared memory when they fit

@@ -5,9 +5,9 @@
 // 810 clocks (five dependent shuffle + DADD, ~120 clocks each, measured on one
 // warp).  A warp reduction of a 32-bit integer (redux.sync) takes 45.  The
 // sums here are therefore formed in fixed point: each addend p is placed in a
-// 96-bit window below a bound 2^E known beforehand (|p| < 2^E, by
-// Cauchy-Schwarz from the norms of the vectors that are dotted), cut into four
-// signed 24-bit pieces, and the pieces are summed as integers: over a warp by
+// 96-bit window below a bound 2^E (|p| < 2^E, by Cauchy-Schwarz from the norms
+// of the vectors that are dotted, where they are known), cut into four signed
+// 24-bit pieces, and the pieces are summed as integers: over a warp by
 // four redux.sync, over a block and over the grid as two 64-bit limbs.
 //
 // The window holds every addend above 2^(E-43) exactly and cuts the others at
@@ -16,8 +16,8 @@
 // atomics instead of publishing partials that every block has to read back and
 // add up.  That is more accurate than FP64 additions while the sum's largest
 // addends are near the bound, and less where all of them are far below it: the
-// callers look at how far.  An addend outside the window (Inf, NaN, or a bound that does not
-// hold) is reported by the return value; the callers turn the sum into NaN.
+// callers look at how far.  An addend outside the window (Inf, NaN, or a bound
+// that does not hold) is reported by the return value, and the sum is not taken.
 #pragma once
 
 #include "common.cuh"

@@ -296,12 +296,14 @@ PSF_DEVINL void lz_persist_body(KState& st, const CsrDev& A, int i_begin, int i_
     // start of the SpMV phase by a lane of the producer warp, which has tiles
     // in flight then: the consumer warps do not wait for it.
     if (threadIdx.x == kConsumerWarps * 32 + 1) {
-      if (kMon && bid == 0) *(volatile long long*)(words + (i % 3) * kLzBuf + 2) = 2ll * i + (*(volatile int*)&c->stop_req != 0);
+      if (kMon && bid == 0)
+        *(volatile long long*)(words + (i % 3) * kLzBuf + 2) = 2ll * i + (*(volatile int*)&c->stop_req != 0);
       if (i > i_begin) {
         sc = 1.0 / ldexp(sm.scal[5], k2);
         if (bid == 0) st.s[i] = sc;
         // the window, from alpha and beta of the previous step (zeros tell nothing)
-        const unsigned m = max((unsigned)__double2hiint(sm.scal[2]) & 0x7fffffffu, (unsigned)__double2hiint(sm.scal[3]));
+        const unsigned m =
+            max((unsigned)__double2hiint(sm.scal[2]) & 0x7fffffffu, (unsigned)__double2hiint(sm.scal[3]));
         if (m > 0xfffffu) sm.window = (int)(m >> 20) - 1022 + kLzNext;
       }
       sm.scal[0] = sc;

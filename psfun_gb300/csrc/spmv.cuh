@@ -38,7 +38,7 @@ struct CsrDev {
   int32_t ntiles;
   unsigned* sched;  // [0] next tile, [1] blocks done: zero between launches
   const int2* __restrict__ tile_desc;  // {first row, first stored entry} per tile (+1 sentinel)
-  const uint16_t* __restrict__ order;  // rows of every tile by descending length, or null: not staged (see k_tile_order)
+  const uint16_t* __restrict__ order;  // rows of every tile by descending length (k_tile_order); null: not staged
   int stream;  // matrix larger than half of L2: stage tiles with an L2 evict-first policy
 };
 

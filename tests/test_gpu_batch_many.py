@@ -58,7 +58,8 @@ def test_estimates_handed_to_the_steps(lib, count, R, itmax, t, eps):
     for k in range(count):
         A = matrices.laplacian_2d(19 + k % 7)
         X = torch.as_tensor(np.random.default_rng(k).standard_normal((R, A.shape[0])), device="cuda")
-        items.append((A, pg.CsrMatrix.from_scipy(sp.csr_matrix(A)), X, torch.empty_like(X), t * (0.4 + 0.6 * (k % 5) / 5)))
+        items.append((A, pg.CsrMatrix.from_scipy(sp.csr_matrix(A)), X, torch.empty_like(X),
+                      t * (0.4 + 0.6 * (k % 5) / 5)))
     _, infos, iters, errs = pg.krylov_batch(meth, fun, [i[1:] for i in items], eps, itmax=itmax, istop=1)
     infos, iters, errs = (np.reshape(v, (count, R)) for v in (infos, iters, errs))
     assert not infos.any()
