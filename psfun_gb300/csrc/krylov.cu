@@ -306,6 +306,12 @@ PSF_DEVINL void lz_persist_body(KState& st, const CsrDev& A, int i_begin, int i_
             max((unsigned)__double2hiint(sm.scal[2]) & 0x7fffffffu, (unsigned)__double2hiint(sm.scal[3]));
         if (m > 0xfffffu) sm.window = (int)(m >> 20) - 1022 + kLzNext;
       }
+      // the next step's words: every CTA has read what they held two steps ago
+      // (this one has the sum of the last, which all posted after that), and
+      // adds to them after this CTA's post of the norm
+      if (bid == 0)
+#pragma unroll
+        for (int q = 0; q < kLzUsed; ++q) words[((i + 1) % 3) * kLzBuf + q] = lz_word_start(q);
       sm.scal[0] = sc;
       sm.scal[1] = (i >= 2) ? beta_i * sprev / sc : 0.0;
     }
@@ -348,11 +354,6 @@ PSF_DEVINL void lz_persist_body(KState& st, const CsrDev& A, int i_begin, int i_
         sm.scal[2] = a;
         sm.scal[4] = stop;
         sm.scal[6] = up ? 0.0 : 1.0;
-        // the next step's words: every CTA has read what they held two steps
-        // ago, and adds to them after this CTA's next post
-        if (bid == 0)
-#pragma unroll
-          for (int q = 0; q < kLzUsed; ++q) words[((i + 1) % 3) * kLzBuf + q] = lz_word_start(q);
         if (bid == 0 && stop == 0.0) {
           HAT(st, i, i) = a;
           if (i >= 2) c->itx = i - 1;
